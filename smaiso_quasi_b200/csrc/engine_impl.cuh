@@ -168,14 +168,13 @@ class Engine : public EngineBase {
       const int rc = autotune();
       if (rc) return rc;
     } else if (cfg_.autotune == 2) {   // every warp-tile candidate (tests of those kernels)
-      tune_.zwarp[0] = tune_.zwarp[1] = true;
       for (auto& a : tune_.xywarp) a[0] = a[1] = true;
     }
     return capture();
   }
 
   // Time each tunable pass's candidate kernels on the scratch fields (zeros)
-  // and keep the fastest: the z pass as CTA or warp tiles, per type; in the
+  // and keep the fastest: the x and y passes as CTA or warp tiles, per type; in the
   // BF16X3 form the plain x and y passes on the tensor cores or by FFT.  The
   // two candidates are timed in alternation (5 rounds of 10 launches each, the
   // best round of each counts), and the default stays unless the other is
@@ -233,17 +232,10 @@ class Engine : public EngineBase {
       return alt < 0.97f * cur ? !dflt : dflt;
     };
     Tuning best = tune_;
-    // z pass, storage type and (FP32 form) double
+    // storage type and (FP32 form) double
     for (int d = 0; d < (kStateCopy<T> ? 2 : 1); ++d) {
       const int slot = kStateCopy<T> ? d : 1;
       float ms[2];
-      auto z = [&]() -> cudaError_t {
-        if (d == 0) return launch_zpass<T>(g_, E01, tb_.t[2], c_.tmp, c_.tmp, stream_);
-        return launch_zpass<double>(g_, E01, tb64_.t[2], c_.tmp64, c_.tmp64, stream_);
-      };
-      if (!race([&](int v) { tune_.zwarp[slot] = v == 1; }, z, ms)) return QUASI_ERR_CUDA;
-      best.zwarp[slot] = better(ms, Tuning{}.zwarp[slot]);
-      tune_ = best;
       // x and y passes as CTA or warp tiles (the plain pass decides for all
       // passes of that axis and type)
       for (int a = 0; a < 2; ++a) {
@@ -470,8 +462,8 @@ class Engine : public EngineBase {
   void note_steps(int n) override { nloop_ += n; }
   bool initialized() const override { return initialized_; }
   void tuning(int out[4]) const override {
-    for (int d = 0; d < 2; ++d)
-      out[d] = int(tune_.zwarp[d]) | (int(tune_.xywarp[0][d]) << 1) | (int(tune_.xywarp[1][d]) << 2);
+    for (int d = 0; d < 2; ++d)   // z passes always run as warp tiles (row_pass.cuh)
+      out[d] = 1 | (int(tune_.xywarp[0][d]) << 1) | (int(tune_.xywarp[1][d]) << 2);
     out[2] = tc_on_ ? tune_.tc_axes : 0;
     out[3] = tune_.measured;
   }
@@ -617,8 +609,6 @@ class Engine : public EngineBase {
     t.enabled = true;
     t.tc = tc_on_ ? &tc_tables_ : nullptr;
     t.tc_axes = tune_.tc_axes;
-    t.zwarp[0] = tune_.zwarp[0];
-    t.zwarp[1] = tune_.zwarp[1];
     for (int a = 0; a < 2; ++a)
       for (int d = 0; d < 2; ++d) t.xywarp[a][d] = tune_.xywarp[a][d];
   }
@@ -751,7 +741,6 @@ class Engine : public EngineBase {
   bool tc_on_ = false;
   // the autotuner's choices (see autotune())
   struct Tuning {
-    bool zwarp[2] = {false, true};
     bool xywarp[2][2] = {{false, false}, {false, false}};   // [axis x, y][float, double]
     int tc_axes = 3;
     bool measured = false;

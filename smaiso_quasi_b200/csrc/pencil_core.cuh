@@ -1,0 +1,297 @@
+// Transforms of pencils held in registers: the building block of the z passes
+// (rows, row_pass.cuh), the x / y passes (columns, col_pass.cuh) and of the
+// stages fused between them.
+//
+// L lanes share one complex pencil (two adjacent real pencils of the field, the
+// real and the imaginary part).  Lane l holds the elements k = l + L t,
+// t < E = N / L, before and after every radix stage: a Stockham stage of radix R
+// reads e = b + t N/R with b = l + L c, which is that set, and the last stage
+// writes it.  Only the writes in between are scattered; they go through an
+// exchange buffer in shared memory and are read back in order, so a transform
+// costs (stages - 1) shared-memory round trips and nothing else (the tile
+// transforms of r2r_core.cuh stage their input and output as well and read the
+// input twice).
+//
+// The pairing (k, N - k) of the inverse pre-twiddle and of the forward unpack is
+// lane l against lane (L - l) mod L: shuffles.  Kinds and Makhoul's permutation
+// are those of r2r_core.cuh.
+//
+// `W` places a pencil's lanes: l(), partner() (the lane of the warp that holds
+// l' = (L - l) mod L of the same pencil), at(e) (element e of this pencil in the
+// exchange buffer), shfl(value, lane) and sync() (all lanes of the exchange
+// buffer).  A test runs the same code with host threads as lanes.
+#pragma once
+#include "r2r_core.cuh"
+
+namespace quasi {
+
+template <typename T> struct Dft<T, 12> {
+  // 4 x 3 split: X[k1 + 4 k2] = sum_n2 W_3^{n2 k2} W_12^{n2 k1} sum_n1 a[3 n1 + n2] W_4^{n1 k1}
+  QHD static void run(Cx<T>* a) {
+    const T h = T(0.5), s = T(0.86602540378443864676372317075294);
+    Cx<T> t[3][4];
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) {
+#pragma unroll
+      for (int n1 = 0; n1 < 4; ++n1) t[n2][n1] = a[3 * n1 + n2];
+      Dft<T, 4>::run(t[n2]);
+    }
+    t[1][1] = cmul(t[1][1], Cx<T>{s, -h});
+    t[1][2] = cmul(t[1][2], Cx<T>{h, -s});
+    t[1][3] = mul_mi(t[1][3]);
+    t[2][1] = cmul(t[2][1], Cx<T>{h, -s});
+    t[2][2] = cmul(t[2][2], Cx<T>{-h, -s});
+    t[2][3] = Cx<T>{-t[2][3].x, -t[2][3].y};
+#pragma unroll
+    for (int k1 = 0; k1 < 4; ++k1) {
+      Cx<T> u[3] = {t[0][k1], t[1][k1], t[2][k1]};
+      Dft<T, 3>::run(u);
+#pragma unroll
+      for (int k2 = 0; k2 < 3; ++k2) a[k1 + 4 * k2] = u[k2];
+    }
+  }
+};
+
+// Lanes per pencil and radices: the first radix is E = N / L, and every stage's
+// N / R butterflies are a multiple of L.
+struct RowPlan {
+  int lanes, n_stages, r[3];
+};
+QHD constexpr RowPlan row_plan(int n) {
+  switch (n) {
+    case 8: return {4, 3, {2, 2, 2}};
+    case 16: return {4, 2, {4, 4, 0}};
+    case 32: return {4, 2, {8, 4, 0}};
+    case 64: return {8, 2, {8, 8, 0}};
+    case 96: return {8, 3, {12, 4, 2}};
+    case 128: return {8, 2, {16, 8, 0}};
+    case 192: return {16, 3, {12, 4, 4}};
+    case 256: return {16, 2, {16, 16, 0}};
+    case 512: return {32, 3, {16, 8, 4}};
+    default: return {0, 0, {0, 0, 0}};
+  }
+}
+
+template <typename T, int N>
+struct PencilFFT {
+  static constexpr RowPlan plan = row_plan(N);
+  static_assert(plan.lanes > 0, "unsupported transform length");
+  static constexpr int L = plan.lanes, E = N / L, H = E / 2;
+  static constexpr int R1 = plan.r[0];
+  static_assert(R1 == E && E % 2 == 0, "the first radix is a lane's share");
+  // padded place of element e: the first stage writes with stride R1
+  QHD static constexpr int phi(int e) { return e + e / R1; }
+  static constexpr int kPadded = N - 1 + (N - 1) / R1 + 1;
+  // tables in shared memory, per CTA: the first stage's twiddles W_N^{l u} as
+  // [u][l], the quarter-wave table, and W_N^t when there is a third stage
+  static constexpr int kTables = plan.n_stages > 2 ? 3 : 2;
+  struct Tab {
+    const Cx<T>*tw1, *quarter, *root;
+  };
+  static constexpr size_t table_bytes() { return size_t(kTables) * N * sizeof(Cx<T>); }
+  // fills the tables at `t` (kTables * N entries); the caller synchronises
+  QHD static Tab fill_tables(Cx<T>* t, Tables<T> tb, int tid, int nt) {
+    for (int e = tid; e < N; e += nt) {
+      t[e] = tb.root[(e / L) * (e % L)];
+      t[N + e] = tb.quarter[e];
+      if (kTables > 2) t[2 * N + e] = tb.root[e];
+    }
+    return Tab{t, t + N, t + 2 * N};
+  }
+
+  // One stage and (unless it is the last) the exchange after it.
+  template <int ST, class W>
+  QHD static void stage(const W& w, Cx<T>* v, Cx<T>* xb, const Tab& tb) {
+    constexpr int R = plan.r[ST], B = E / R;
+    constexpr int s = ST == 0 ? 1 : ST == 1 ? plan.r[0] : plan.r[0] * plan.r[1];
+    constexpr bool last = ST == plan.n_stages - 1;
+    const int l = w.l();
+#pragma unroll
+    for (int c = 0; c < B; ++c) {
+      Cx<T> a[R];
+#pragma unroll
+      for (int u = 0; u < R; ++u) a[u] = v[c + B * u];
+      Dft<T, R>::run(a);
+      if constexpr (last) {
+#pragma unroll
+        for (int u = 0; u < R; ++u) v[c + B * u] = a[u];
+      } else {
+        const int b = l + L * c, p = b / s, q = b - p * s;
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+          Cx<T> f = a[u];
+          if (u) f = cmul(f, ST == 0 ? tb.tw1[u * L + l] : tb.root[s * p * u]);
+          xb[w.at(q + s * (R * p + u))] = f;
+        }
+      }
+    }
+    if constexpr (!last) {
+      w.sync();
+#pragma unroll
+      for (int t = 0; t < E; ++t) v[t] = xb[w.at(l + L * t)];
+      w.sync();
+    }
+  }
+  template <class W>
+  QHD static void dft(const W& w, Cx<T>* v, Cx<T>* xb, const Tab& tb) {
+    stage<0>(w, v, xb, tb);
+    stage<1>(w, v, xb, tb);
+    if constexpr (plan.n_stages > 2) stage<2>(w, v, xb, tb);
+  }
+
+  // Inverse kinds (REDFT01; RODFT01 with its input reversed by the caller):
+  // v[t] = (y_k of row a, y_k of row b) -> F_k, the complex DFT whose conjugate
+  // holds the permuted outputs.  v_k = quarter_k ((a_k + b_{N-k}) + i (a_{N-k} - b_k)).
+  template <class W>
+  QHD static void inverse(const W& w, Cx<T>* v, Cx<T>* xb, const Tab& tb) {
+    const int l = w.l(), src = w.partner();
+    Cx<T> prev = {T(0), T(0)};   // lane 0: y_N = 0, then its element E - t
+#pragma unroll
+    for (int t = 0; t < H; ++t) {
+      const int u = E - 1 - t;
+      const Cx<T> lo = v[t], hi = v[u], up = v[t + 1];
+      const Cx<T> plo = w.shfl(l ? hi : prev, src), phi_ = w.shfl(l ? lo : up, src);
+      prev = hi;
+      v[t] = cmul(tb.quarter[l + L * t], Cx<T>{lo.x + plo.y, plo.x - lo.y});
+      v[u] = cmul(tb.quarter[l + L * u], Cx<T>{hi.x + phi_.y, phi_.x - hi.y});
+    }
+    dft(w, v, xb, tb);
+  }
+
+  // Forward kinds (REDFT10; RODFT10 with odd positions negated and its output
+  // reversed by the caller): v[t] = the permuted input -> v[t] = (y_k of row a,
+  // y_k of row b).
+  template <class W>
+  QHD static void forward(const W& w, Cx<T>* v, Cx<T>* xb, const Tab& tb) {
+    dft(w, v, xb, tb);
+    const int l = w.l(), src = w.partner();
+    Cx<T> prev = v[0];   // lane 0: Z_N = Z_0
+#pragma unroll
+    for (int t = 0; t < H; ++t) {
+      const int u = E - 1 - t;
+      const Cx<T> lo = v[t], hi = v[u], up = v[t + 1];
+      const Cx<T> plo = w.shfl(l ? hi : prev, src), phi_ = w.shfl(l ? lo : up, src);
+      prev = hi;
+      v[t] = unpack(lo, plo, tb.quarter[l + L * t]);
+      v[u] = unpack(hi, phi_, tb.quarter[l + L * u]);
+    }
+  }
+  // y_k of both rows from Z_k and Z_{N-k}
+  QHD static Cx<T> unpack(Cx<T> z, Cx<T> n, Cx<T> q) {
+    return Cx<T>{q.x * (z.x + n.x) - q.y * (z.y - n.y), q.x * (z.y + n.y) + q.y * (z.x - n.x)};
+  }
+
+  // Position of y_k along the axis.  sine: the kind's own order (k reversed);
+  // mode (sine only): by mode number N - k, where the top mode N (k = 0) has no
+  // place and the caller takes it as zero.
+  QHD static int spec(int k, bool sine, bool mode = false) { return !sine ? k : mode ? (k ? N - k : 0) : N - 1 - k; }
+  // Position of the permuted element k: even positions first, then the odd ones
+  // from the top (sine kinds: odd positions negated).
+  QHD static int pos(int k) { return k < N / 2 ? 2 * k : 2 * (N - 1 - k) + 1; }
+};
+
+// Rows: pencils of 2 rows, 32 / L pencils per warp.  Makhoul's permutation maps
+// k < N/2 to position 2k and k >= N/2 to 2 (N - 1 - k) + 1, so the pair of
+// adjacent positions (n, n + 1), n = 2 l + 2 L t, is this lane's element t and
+// lane L - 1 - l's element E - 1 - t: one shuffle gives each lane adjacent pairs
+// of both rows, and every real-space access is a 2-element vector.
+template <typename T, int N>
+struct RowFFT : PencilFFT<T, N> {
+  using P = PencilFFT<T, N>;
+  using P::E;
+  using P::H;
+  using P::L;
+  static constexpr int PPW = 32 / L, ROWS = 2 * PPW;   // pencils and rows of a warp
+  // complex elements between the pencils of a warp: the lanes of one access
+  // phase (16 in float, 8 in double) that span several pencils hit distinct banks
+  static constexpr int pencil_stride() {
+    constexpr int ph = sizeof(T) == 8 ? 8 : 16;
+    int x = P::kPadded;
+    if (L < ph)
+      while (x % ph != L) ++x;
+    return x;
+  }
+  static constexpr int XS = pencil_stride();
+  static constexpr int XCH = PPW * XS;   // complex elements of a warp's exchange buffer
+  // F_k -> adjacent positions: a[t] = row a at (n, n + 1), b[t] = row b, n = 2 l + 2 L t.
+  // In place: v[t] = row a's pair, v[E - 1 - t] = row b's.  sine: odd positions negated.
+  template <class W>
+  QHD static void to_pairs(const W& w, Cx<T>* v, bool sine) {
+    const int src = w.mirror();
+    const T s = sine ? T(-1) : T(1);
+#pragma unroll
+    for (int t = 0; t < H; ++t) {
+      const Cx<T> o = w.shfl(v[E - 1 - t], src), e = v[t];
+      v[t] = Cx<T>{e.x, s * o.x};
+      v[E - 1 - t] = Cx<T>{-e.y, -s * o.y};
+    }
+  }
+  // the reverse, for a forward kind's input
+  template <class W>
+  QHD static void from_pairs(const W& w, Cx<T>* v, bool sine) {
+    const int src = w.mirror();
+    const T s = sine ? T(-1) : T(1);
+#pragma unroll
+    for (int t = 0; t < H; ++t) {
+      const Cx<T> a = v[t], b = v[E - 1 - t];
+      v[t] = Cx<T>{a.x, b.x};
+      v[E - 1 - t] = w.shfl(Cx<T>{s * a.y, s * b.y}, src);
+    }
+  }
+
+};
+
+#ifdef __CUDACC__
+// The lanes of a warp as RowFFT places them.
+template <typename T, int N>
+struct RowWarp {
+  using F = RowFFT<T, N>;
+  int lane;
+  __device__ __forceinline__ int l() const { return lane % F::L; }
+  __device__ __forceinline__ int pencil() const { return lane / F::L; }
+  __device__ __forceinline__ int partner() const { return lane - l() + ((F::L - l()) & (F::L - 1)); }
+  __device__ __forceinline__ int mirror() const { return lane + F::L - 1 - 2 * l(); }
+  __device__ __forceinline__ int at(int e) const { return pencil() * F::XS + F::phi(e); }
+  __device__ __forceinline__ void sync() const { __syncwarp(); }
+  __device__ __forceinline__ Cx<T> shfl(Cx<T> v, int src) const {
+    return Cx<T>{__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)};
+  }
+};
+
+// Columns: a tile of G pencils (2 G adjacent k) along the x or y axis on
+// THREADS = G L threads (whole warps).  A warp holds S = 32 / G values of l for
+// all G pencils, chosen so that l and L - l share it (the partner stays a
+// shuffle): l and L - l for l in [w S / 2, (w + 1) S / 2), with L / 2 beside 0.
+// Neighbouring l differ in parity, which puts a half-warp's float accesses to
+// the exchange rows [e][g] on distinct banks.  Tiles of one warp synchronise the
+// warp, wider ones a named barrier.
+template <int N, int G>
+struct ColTile {
+  static constexpr int L = row_plan(N).lanes, R1 = N / L, S = 32 / G;
+  static constexpr int THREADS = G * L;
+  static_assert(THREADS % 32 == 0 && S >= 2, "a tile is whole warps");
+  static constexpr int ROWS = N - 1 + (N - 1) / R1 + 1;   // padded rows of G of the exchange buffer
+  static constexpr int XCH = ROWS * G;                    // its complex elements
+  int ll, part, g, bar;
+  // r: thread of the tile; bar: its named barrier
+  __device__ __forceinline__ ColTile(int r, int barrier) : bar(barrier) {
+    const int lane = r & 31, sub = lane / G, h = sub % (S / 2), lo = (r / 32) * (S / 2) + h;
+    g = lane % G;
+    ll = sub < S / 2 ? lo : (lo == 0 ? L / 2 : L - lo);
+    part = (lo == 0 ? sub : sub ^ (S / 2)) * G + g;
+  }
+  __device__ __forceinline__ int l() const { return ll; }
+  __device__ __forceinline__ int partner() const { return part; }
+  __device__ __forceinline__ int at(int e) const { return (e + e / R1) * G + g; }
+  __device__ __forceinline__ void sync() const {
+    if constexpr (THREADS == 32) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(THREADS) : "memory");
+  }
+  template <typename T>
+  __device__ __forceinline__ Cx<T> shfl(Cx<T> v, int src) const {
+    return Cx<T>{__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)};
+  }
+};
+#endif
+
+}  // namespace quasi

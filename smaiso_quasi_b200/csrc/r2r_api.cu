@@ -31,8 +31,6 @@ struct R2RBase {
     t.poll_limit = inject_polls;
     t.tc = tc_on ? &tc_tables : nullptr;
     t.tc_axes = 3;
-    t.zwarp[0] = false;
-    t.zwarp[1] = true;
   }
   void end_tma() {   // the injection lasts one execution
     TmaConfig& t = tma_config();

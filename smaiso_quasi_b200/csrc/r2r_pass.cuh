@@ -17,14 +17,11 @@
 #include <type_traits>
 
 #include "r2r_core.cuh"
+#include "row_pass.cuh"
 #include "tc_pass.cuh"
 #include "tma.cuh"
 
 namespace quasi {
-
-template <typename T> struct Vec2;
-template <> struct Vec2<float> { using type = float2; };
-template <> struct Vec2<double> { using type = double2; };
 
 struct DevExec {
   template <class R, class W, class Regs>
@@ -48,10 +45,6 @@ struct WarpExec {
     if (after) __syncwarp();
   }
   __device__ __forceinline__ void sync() { __syncwarp(); }
-};
-
-struct Geom {
-  int nx, ny, nz;
 };
 
 // ---------------------------------------------------------------------------
@@ -806,9 +799,6 @@ struct TmaConfig {
   uint32_t poll_limit = kTmaPollLimit;   // polls before a tile wait gives up
   int skip_tile = -1;     // fault injection: a tile whose copy is never issued
   const tc::Tables4* tc = nullptr;   // split-BF16 form: plain float x / y passes on the tensor cores
-  // z passes of length 64..256 as warp tiles (tma_zpass_warp_kernel) rather
-  // than CTA tiles, for float [0] and double [1] passes
-  bool zwarp[2] = {false, true};
   // x [0] / y [1] passes as warp tiles (tma_pass_warp_kernel), float / double
   bool xywarp[2][2] = {{false, false}, {false, false}};
   int tc_axes = 3;        // with tc: the axes (bit 0 x, bit 1 y) that use it

@@ -23,7 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "r2r_pass.cuh"
-#include "z_pass.cuh"
+#include "row_pass.cuh"
 
 namespace quasi {
 
@@ -625,6 +625,13 @@ struct AxisTables {
   Tables<T> t[3];
 };
 
+// z pass src -> dst on this thread's configuration (row_pass.cuh).
+template <typename T>
+cudaError_t launch_zpass(const Geom& g, int kind, Tables<T> tb, const T* src, T* dst, cudaStream_t s, int ks = 0,
+                         const T* mk = nullptr) {
+  return launch_row_pass<T>(g, kind, tb, src, dst, ks, mk, tma_config().sms, tma_config().zrev, s);
+}
+
 // y and z passes of `src` (plain field) into `st` (the y pass in place, the
 // z pass into st.dst).  kshift = 1: the z pass transforms row[k + 1] (zero at
 // the top) in place of row[k], the z shift of a z gradient
@@ -728,7 +735,7 @@ inline dim3 row_block(int nz) {
 #define QUASI_EW(kern, ...) kern<<<ew_grid(kern, 256), 256, 0, s>>>(__VA_ARGS__)
 #define QUASI_EW_ON(kern, strm, ...) kern<<<ew_grid(kern, 256), 256, 0, strm>>>(__VA_ARGS__)
 
-// z pass src -> dst: the TMA z kernel, else the general pass.  ks = 1
+// z pass src -> dst: the row kernel, else the general pass.  ks = 1
 // transforms row[k + 1] (zero at the top), ks = 2 -mk[k] row[k + 1].
 template <typename T>
 cudaError_t zpass(const Geom& g, int kind, Tables<T> tb, T* src, T* dst, cudaStream_t s, int ks = 0,
