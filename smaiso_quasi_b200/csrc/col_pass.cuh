@@ -1,0 +1,757 @@
+// Passes along the x and y axes on tiles of G pencils x all N rows, the pencils
+// in registers (pencil_core.cuh, ColTile): rows are loaded and stored directly
+// (2 G adjacent k per row: 64 to 128 bytes), one exchange through shared memory
+// in between.  Everything that a field goes through between two y passes runs in
+// one kernel:
+//   col_batch_kernel   the passes of several fields along one axis in one launch
+//   density_x_kernel   rho: forward x, the density filter, every inverse x pass
+//                      taken from rho^
+//   update_x_kernel    N: forward x, the semi-implicit update, every inverse x
+//                      pass taken from the new psi^
+//   project_x_kernel   the stress and divv: forward x, pressure and velocity
+//                      projection, inverse x
+//
+// Sine spectra between passes are stored by mode number: place m holds mode m
+// (place 0 is zero, the top mode N, which nothing reads, has no place).  The
+// reference keeps mode m at index m - 1 (quasi.cpp:397-431), so that every term
+// that couples a sine and a cosine spectrum reads a neighbour; by mode number it
+// is local, and the projection needs no neighbouring tile.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "row_pass.cuh"
+
+namespace quasi {
+
+__device__ __forceinline__ double rcp(double x) { return __drcp_rn(x); }
+// FP32: the hardware reciprocal (within 2 ulp, below the FP32 storage rounding)
+__device__ __forceinline__ float rcp(float x) { return __fdividef(1.0f, x); }
+
+// Keeps the compiler from hoisting the E row offsets of a tile (64 bits each)
+// out of the tile loop, where they spill.
+__device__ __forceinline__ int opaque(int x) {
+  asm volatile("" : "+r"(x));
+  return x;
+}
+
+// The tile's columns in a field along one axis: element (n, this lane's pair).
+struct ColGeom {
+  int stride;      // elements between rows along the axis
+  int kt;          // tiles per outer index
+  size_t outer;    // elements between outer indices
+};
+template <int AXIS, int G>
+__host__ __device__ __forceinline__ ColGeom col_geom(const Geom& g) {
+  if (AXIS == 1) return {g.nz, g.nz / (2 * G), size_t(g.ny) * g.nz};
+  return {g.ny * g.nz, g.nz / (2 * G), size_t(g.nz)};
+}
+template <int AXIS>
+inline int col_tiles(const Geom& g, int G) { return (AXIS == 1 ? g.nx : g.ny) * (g.nz / (2 * G)); }
+
+// The threads of a tile start fetching its N rows of 2 G elements into L2.
+template <class C, int N, int G, typename T>
+__device__ __forceinline__ void prefetch_tile(const T* a, int stride, int r) {
+  for (int n = r; n < N; n += C::THREADS) prefetch_l2(a + unsigned(n * stride), 2 * G * sizeof(T));
+}
+
+// How a spectral position is read or written along the axis.
+//   cosine: place k.  sine by mode: element k is mode N - k, element 0 nothing.
+template <typename T, int N>
+struct ColIO {
+  using F = PencilFFT<T, N>;
+  __device__ __forceinline__ static int place(int k, bool sine) { return F::spec(k, sine, true); }
+  // real positions
+  __device__ __forceinline__ static void load_pos(const T* a, int stride0, int l, Cx<T>* v, bool sine) {
+    const int stride = opaque(stride0);
+    const T s = sine ? T(-1) : T(1);
+#pragma unroll
+    for (int t = 0; t < F::E; ++t) {
+      v[t] = ld2(a + unsigned(F::pos(l + F::L * t) * stride));
+      if (t >= F::H) v[t] = cscale(v[t], s);
+    }
+  }
+  // an inverse's output (b, a), odd positions negated for sine kinds
+  __device__ __forceinline__ static void store_pos(T* a, int stride0, int l, const Cx<T>* v, bool sine) {
+    const int stride = opaque(stride0);
+    const T s = sine ? T(-1) : T(1);
+#pragma unroll
+    for (int t = 0; t < F::E; ++t) {
+      const Cx<T> u = t < F::H ? v[t] : cscale(v[t], s);
+      st2(a + unsigned(F::pos(l + F::L * t) * stride), Cx<T>{u.y, u.x});
+    }
+  }
+  // (a branch outside the loop: the positions of either order are then multiples
+  // of the stride from one base)
+  __device__ __forceinline__ static void load_spec(const T* a, int stride0, int l, Cx<T>* v, bool sine) {
+    const int stride = opaque(stride0);
+    if (!sine) {
+#pragma unroll
+      for (int t = 0; t < F::E; ++t) v[t] = ld2(a + unsigned((l + F::L * t) * stride));
+    } else {
+#pragma unroll
+      for (int t = 0; t < F::E; ++t) {
+        const int k = l + F::L * t, n = t || k ? N - k : 0;
+        v[t] = ld2(a + unsigned(n * stride));
+        if (t == 0 && k == 0) v[t] = Cx<T>{T(0), T(0)};
+      }
+    }
+  }
+  __device__ __forceinline__ static void store_spec(T* a, int stride0, int l, const Cx<T>* v, bool sine) {
+    const int stride = opaque(stride0);
+    if (!sine) {
+#pragma unroll
+      for (int t = 0; t < F::E; ++t) st2(a + unsigned((l + F::L * t) * stride), v[t]);
+    } else {
+#pragma unroll
+      for (int t = 0; t < F::E; ++t) {
+        const int k = l + F::L * t, n = t || k ? N - k : 0;
+        st2(a + unsigned(n * stride), t == 0 && k == 0 ? Cx<T>{T(0), T(0)} : v[t]);
+      }
+    }
+  }
+};
+
+// ---------------------------------------------------------------------------
+// Passes of several fields
+// ---------------------------------------------------------------------------
+enum ColOp : int {
+  kColCos = 0,    // cosine kind
+  kColSine = 1,   // sine kind, its spectrum by mode number
+  kColGrad = 2,   // (inverse) cosine spectrum c_m -> RODFT01 of the modes -q_m c_m: the derivative along the axis
+  kColBoth = 3    // (inverse) dst = the cosine transform, dst2 = the derivative, one tile load each
+};
+template <typename T>
+struct ColJob {
+  const T* src;
+  T *dst, *dst2;
+  int op;
+};
+constexpr int kMaxJobs = 8;
+template <typename T>
+struct ColJobs {
+  ColJob<T> job[kMaxJobs];
+};
+
+// Pencils of a tile (G): 8, as nz is a multiple of 16; 4 as "warp tiles", which
+// make tiles of the lengths with 8 lanes one warp's own (no barrier).
+// threads of a CTA: at least four warps, one tile per THREADS
+template <int N, int G> constexpr int col_cta() { return ColTile<N, G>::THREADS >= 128 ? ColTile<N, G>::THREADS : 128; }
+
+template <typename T, int N, int G>
+constexpr size_t col_batch_smem() {
+  return PencilFFT<T, N>::table_bytes() + N * sizeof(T) +
+         size_t(col_cta<N, G>() / ColTile<N, G>::THREADS) * ColTile<N, G>::XCH * sizeof(Cx<T>);
+}
+template <typename T, int N, int G, bool FWD>
+__global__ void __launch_bounds__(col_cta<N, G>(), 512 / col_cta<N, G>())
+    col_batch_kernel(const __grid_constant__ ColJobs<T> jobs, int njobs, ColGeom cg, int tiles, Tables<T> tb,
+                     const double* vq, T scale) {
+  using C = ColTile<N, G>;
+  using F = PencilFFT<T, N>;
+  using IO = ColIO<T, N>;
+  constexpr int NT = col_cta<N, G>(), SETS = NT / C::THREADS;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int set = threadIdx.x / C::THREADS;
+  Cx<T>* xb = reinterpret_cast<Cx<T>*>(smem_raw + F::table_bytes()) + set * C::XCH;
+  T* q = reinterpret_cast<T*>(reinterpret_cast<Cx<T>*>(smem_raw + F::table_bytes()) + SETS * C::XCH);
+  const typename F::Tab t = F::fill_tables(reinterpret_cast<Cx<T>*>(smem_raw), tb, threadIdx.x, NT);
+  for (int e = threadIdx.x; e < N; e += NT) q[e] = vq ? T(-vq[e]) : T(0);
+  __syncthreads();
+  const C w(threadIdx.x % C::THREADS, 1 + set);
+  const int l = w.l();
+  for (int x = blockIdx.x * SETS + set; x < tiles * njobs; x += gridDim.x * SETS) {
+    const int j = x / tiles, tile = x - j * tiles;
+    const ColJob<T>& jb = jobs.job[j];
+    auto corner = [&](int i) { return (i / cg.kt) * cg.outer + (i % cg.kt) * 2 * G; };
+    const size_t base = corner(tile) + 2 * w.g;
+    Cx<T> v[F::E];
+    if constexpr (FWD) {
+      const bool sine = jb.op == kColSine;
+      IO::load_pos(jb.src + base, cg.stride, l, v, sine);
+      F::forward(w, v, xb, t);
+      if (scale != T(1)) {
+#pragma unroll
+        for (int i = 0; i < F::E; ++i) v[i] = cscale(v[i], scale);
+      }
+      IO::store_spec(jb.dst + base, cg.stride, l, v, sine);
+    } else {
+      // kColBoth: the derivative first; the tile is read again (from L1 / L2)
+      // before the cosine transform may overwrite it
+#pragma unroll 1
+      for (int pass = jb.op == kColBoth ? 0 : 1; pass < 2; ++pass) {
+        const bool grad = pass == 0 || jb.op == kColGrad, sine = grad || jb.op == kColSine;
+        IO::load_spec(jb.src + base, cg.stride, l, v, sine);
+        if (grad) {
+#pragma unroll
+          for (int i = 0; i < F::E; ++i) v[i] = cscale(v[i], q[IO::place(l + F::L * i, true)]);
+        }
+        F::inverse(w, v, xb, t);
+        IO::store_pos((pass == 0 ? jb.dst2 : jb.dst) + base, cg.stride, l, v, sine);
+      }
+    }
+  }
+}
+
+template <typename T, int N, int G, bool FWD>
+cudaError_t launch_col_batch_g(const Geom& g, int axis, const ColJobs<T>& jobs, int njobs, Tables<T> tb,
+                               const double* vq, T scale, int sms, cudaStream_t s) {
+  constexpr int NT = col_cta<N, G>(), SETS = NT / ColTile<N, G>::THREADS;
+  auto kern = col_batch_kernel<T, N, G, FWD>;
+  static std::atomic<int> cache[kMaxDevices];
+  int per_sm = 1;
+  const cudaError_t e = resident_ctas(kern, NT, col_batch_smem<T, N, G>(), cache, &per_sm);
+  if (e != cudaSuccess) return e;
+  const int tiles = axis == 1 ? col_tiles<1>(g, G) : col_tiles<0>(g, G), work = (tiles * njobs + SETS - 1) / SETS;
+  kern<<<std::min(per_sm * sms, work), NT, col_batch_smem<T, N, G>(), s>>>(
+      jobs, njobs, axis == 1 ? col_geom<1, G>(g) : col_geom<0, G>(g), tiles, tb, vq, scale);
+  return cudaGetLastError();
+}
+template <typename T, int N>
+cudaError_t launch_col_batch_n(const Geom& g, int axis, bool forward, const ColJobs<T>& jobs, int njobs, Tables<T> tb,
+                               const double* vq, T scale, bool narrow, int sms, cudaStream_t s) {
+  if constexpr (row_plan(N).lanes == 8) {
+    if (narrow)
+      return forward ? launch_col_batch_g<T, N, 4, true>(g, axis, jobs, njobs, tb, vq, scale, sms, s)
+                     : launch_col_batch_g<T, N, 4, false>(g, axis, jobs, njobs, tb, vq, scale, sms, s);
+  }
+  return forward ? launch_col_batch_g<T, N, 8, true>(g, axis, jobs, njobs, tb, vq, scale, sms, s)
+                 : launch_col_batch_g<T, N, 8, false>(g, axis, jobs, njobs, tb, vq, scale, sms, s);
+}
+
+// ---------------------------------------------------------------------------
+// x stages.  Per-axis double tables: wavenumbers and density filter factors.
+// ---------------------------------------------------------------------------
+struct XTables {
+  const double *vqx, *vqy, *vqz, *fx, *fy, *fz;
+};
+
+// rho (double, z and y transformed) -> rho^ = scale CT(rho) exp(-1.57^2 q^2 8)
+// (quasi.cpp:1260-1261) -> the x-inverse of rho^ and of its gradient's spectra.
+//   DBL: out0 = x(rho^), out1 = x'(rho^) in double (grad_y, grad_z follow from out0)
+//   else out0 = x(rho^) in double and the three gradient spectra's x passes from
+//   the float copy of rho^, each with its own multiplier (applied before the
+//   transform, so float rounding is not multiplied by the wavenumber)
+// from_spec: take rho^ from memory and leave `in` alone (a loaded state).
+template <typename T>
+struct DensityX {
+  const double* in;
+  double *rhoq, *out0, *out1;
+  T *gx, *gy, *gz;   // float form
+  XTables x;
+  double scale;
+  int from_spec;
+};
+
+// psi^: N -> N^, the semi-implicit update (quasi.cpp:1944-1962,
+// quasi-stb.cpp:1946-1958), then from psi^ the x-inverse passes of the next
+// step: psi and d_x psi in double (grad_y, grad_z share the first), and in T,
+// each with its multiplier, df, lap and the three of grad lap psi (quasi) or
+// -aLin psi^ (stb).
+template <typename T>
+struct UpdateX {
+  const T* in;
+  T *Nq;
+  const T* Nq_old;
+  const double *psiq, *psiq_old;
+  double* psiq_new;
+  double *out0, *out1;
+  T* out[5];
+  XTables x;
+  double ep, alpha, q0, rho_m, dt, scale;
+  const int* nloop;   // steps completed
+  int variant, from_spec;
+};
+
+// Tiles of an x stage: 8 pencils (4 at N = 512), doubles exchanged in halves: a
+// tile then takes 49 KB at N = 256 and four of 4 warps fill an SM (whole exchanges
+// leave room for three: density_x 200 us at 256^3 in the FP32 form against 180;
+// three tiles of 8 warps on 32 lanes per pencil: 217 us, bound by shared memory).
+template <int N> constexpr int x_pencils() { return N >= 512 ? 4 : 8; }
+template <int N, int G> using XTile = ColTile<N, G, false, true>;
+template <int N> constexpr int x_sets() { return 4; }
+// CTAs per SM that the registers must allow
+template <int N>
+constexpr int x_ctas() {
+  return N >= 192 ? 1 : N >= 96 ? 2 : N >= 64 ? 2 : 4;
+}
+template <int N, int G> constexpr int x_cta() { return x_sets<N>() * XTile<N, G>::THREADS; }
+// exchange buffer (double complex, or split: double; and float complex), then the spectrum
+template <int N, int G>
+constexpr size_t x_xch_bytes() { return (size_t(XTile<N, G>::XCH) * (XTile<N, G>::template split<double>() ? 8 : 16) + 15) / 16 * 16; }
+template <int N, int G>
+constexpr size_t x_tile_bytes() { return x_xch_bytes<N, G>() + size_t(N) * G * sizeof(Cx<double>); }
+template <typename T, int N, int G>
+constexpr size_t x_stage_smem() {   // tables of both types, wavenumbers and filter, exchange and spectrum in double
+  return PencilFFT<double, N>::table_bytes() + (sizeof(T) == 4 ? PencilFFT<float, N>::table_bytes() : 0) +
+         2 * N * sizeof(double) + size_t(x_sets<N>()) * x_tile_bytes<N, G>();
+}
+
+// Shared memory of an x stage, as one tile's threads see it.
+template <typename T, int N, int G>
+struct XStage {
+  using C = XTile<N, G>;
+  using F = PencilFFT<T, N>;
+  using FD = PencilFFT<double, N>;
+  static constexpr int NT = x_cta<N, G>();
+  typename FD::Tab td;
+  typename F::Tab tt;
+  double *q, *f;      // wavenumbers and filter factors along x
+  Cx<double>* xd;     // exchange
+  Cx<T>* xt;          // the same bytes for T
+  Cx<double>* spec;   // the tile's spectrum [k][g]
+  __device__ __forceinline__ XStage(unsigned char* sm, int set, Tables<double> tb64, Tables<T> tb, const double* vq,
+                                    const double* fl) {
+    td = FD::fill_tables(reinterpret_cast<Cx<double>*>(sm), tb64, threadIdx.x, NT);
+    sm += FD::table_bytes();
+    if constexpr (sizeof(T) == 4) {
+      tt = F::fill_tables(reinterpret_cast<Cx<T>*>(sm), tb, threadIdx.x, NT);
+      sm += F::table_bytes();
+    } else {
+      tt = td;
+    }
+    q = reinterpret_cast<double*>(sm);
+    f = q + N;
+    for (int e = threadIdx.x; e < N; e += NT) {
+      q[e] = vq[e];
+      f[e] = fl[e];
+    }
+    sm = reinterpret_cast<unsigned char*>(f + N) + set * x_tile_bytes<N, G>();
+    xd = reinterpret_cast<Cx<double>*>(sm);
+    xt = reinterpret_cast<Cx<T>*>(sm);
+    spec = reinterpret_cast<Cx<double>*>(sm + x_xch_bytes<N, G>());
+    __syncthreads();
+  }
+  // the tile's spectrum in T; FP32: the same bytes, after narrow_spectrum()
+  __device__ __forceinline__ Cx<T>* spect() const { return reinterpret_cast<Cx<T>*>(spec); }
+  __device__ __forceinline__ void narrow_spectrum(const C& w) const {
+    if constexpr (sizeof(T) == 4) {
+      Cx<T> y[F::E];
+#pragma unroll
+      for (int t = 0; t < F::E; ++t) {
+        const Cx<double> v = spec[(w.l() + F::L * t) * G + w.g];
+        y[t] = Cx<T>{T(v.x), T(v.y)};
+      }
+      w.sync();
+#pragma unroll
+      for (int t = 0; t < F::E; ++t) spect()[(w.l() + F::L * t) * G + w.g] = y[t];
+      w.sync();
+    }
+  }
+};
+
+template <typename T, int N, int G>
+__global__ void __launch_bounds__(x_cta<N, G>(), x_ctas<N>())
+    density_x_kernel(const __grid_constant__ DensityX<T> a, Geom geom, int tiles, Tables<double> tb64, Tables<T> tb) {
+  using X = XStage<T, N, G>;
+  using C = typename X::C;
+  using F = typename X::F;
+  using FD = typename X::FD;
+  using IO = ColIO<T, N>;
+  using IOD = ColIO<double, N>;
+  constexpr bool kDbl = sizeof(T) == 8;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int set = threadIdx.x / C::THREADS;
+  const X sh(smem_raw, set, tb64, tb, a.x.vqx, a.x.fx);
+  const C w(threadIdx.x % C::THREADS, 1 + set);
+  const int l = w.l();
+  const ColGeom cg = col_geom<0, G>(geom);
+  for (int tile = blockIdx.x * x_sets<N>() + set; tile < tiles; tile += gridDim.x * x_sets<N>()) {
+    const int j = tile / cg.kt, k0 = (tile - j * cg.kt) * 2 * G + 2 * w.g;
+    const size_t base = j * cg.outer + k0;
+    const double qy = a.x.vqy[j], qz0 = a.x.vqz[k0], qz1 = a.x.vqz[k0 + 1];
+    if (const int nt = tile + gridDim.x * x_sets<N>(); nt < tiles && !a.from_spec)
+      prefetch_tile<C, N, G>(a.in + (nt / cg.kt) * cg.outer + (nt % cg.kt) * 2 * G, opaque(cg.stride),
+                                  threadIdx.x % C::THREADS);
+    Cx<double> v[FD::E];
+    if (!a.from_spec) {
+      IOD::load_pos(a.in + base, cg.stride, l, v, false);
+      FD::forward(w, v, sh.xd, sh.td);
+      const double fy = a.x.fy[j], fz0 = a.x.fz[k0], fz1 = a.x.fz[k0 + 1];
+#pragma unroll
+      for (int t = 0; t < FD::E; ++t) {
+        const double fx = sh.f[l + FD::L * t];
+        v[t] = Cx<double>{a.scale * v[t].x * (fx * fy * fz0), a.scale * v[t].y * (fx * fy * fz1)};
+      }
+      IOD::store_spec(a.rhoq + base, cg.stride, l, v, false);
+    } else {
+      IOD::load_spec(a.rhoq + base, cg.stride, l, v, false);
+    }
+#pragma unroll
+    for (int t = 0; t < FD::E; ++t) sh.spec[(l + FD::L * t) * G + w.g] = v[t];
+    w.sync();
+#pragma unroll 1
+    for (int o = 0; o < (kDbl ? 2 : 1); ++o) {
+#pragma unroll
+      for (int t = 0; t < FD::E; ++t) {
+        const int k = l + FD::L * t, n = IOD::place(k, o == 1);
+        v[t] = sh.spec[n * G + w.g];
+        if (o == 1) v[t] = cscale(v[t], -sh.q[n]);   // (mode 0: q = 0)
+      }
+      FD::inverse(w, v, sh.xd, sh.td);
+      IOD::store_pos((o ? a.out1 : a.out0) + base, cg.stride, l, v, o == 1);
+    }
+    if constexpr (!kDbl) {
+      sh.narrow_spectrum(w);
+      const T mq[3] = {T(0), T(-qy), T(-qz0)}, mq1 = T(-qz1);
+#pragma unroll 1
+      for (int o = 0; o < 3; ++o) {
+        Cx<T> u[F::E];
+#pragma unroll
+        for (int t = 0; t < F::E; ++t) {
+          const int n = IO::place(l + F::L * t, o == 0);
+          const Cx<T> y = sh.spect()[n * G + w.g];
+          const T m0 = o == 0 ? T(-sh.q[n]) : o == 1 ? mq[1] : mq[2], m1 = o == 2 ? mq1 : m0;
+          u[t] = Cx<T>{y.x * m0, y.y * m1};
+        }
+        F::inverse(w, u, sh.xt, sh.tt);
+        IO::store_pos((o == 0 ? a.gx : o == 1 ? a.gy : a.gz) + base, cg.stride, l, u, o == 0);
+      }
+    }
+    w.sync();   // the next tile rewrites the spectrum
+  }
+}
+
+template <typename T, int N, int G>
+__global__ void __launch_bounds__(x_cta<N, G>(), x_ctas<N>())
+    update_x_kernel(const __grid_constant__ UpdateX<T> a, Geom geom, int tiles, Tables<double> tb64, Tables<T> tb) {
+  using X = XStage<T, N, G>;
+  using C = typename X::C;
+  using F = typename X::F;
+  using FD = typename X::FD;
+  using IO = ColIO<T, N>;
+  using IOD = ColIO<double, N>;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int set = threadIdx.x / C::THREADS;
+  const X sh(smem_raw, set, tb64, tb, a.x.vqx, a.x.vqx);
+  const C w(threadIdx.x % C::THREADS, 1 + set);
+  const int l = w.l();
+  const bool quasi = a.variant == 0, first = *a.nloop == 0;
+  const ColGeom cg = col_geom<0, G>(geom);
+  const double dtd2 = a.dt / 2, dsc = dtd2 * a.scale, q02 = a.q0 * a.q0;
+  for (int tile = blockIdx.x * x_sets<N>() + set; tile < tiles; tile += gridDim.x * x_sets<N>()) {
+    const int j = tile / cg.kt, k0 = (tile - j * cg.kt) * 2 * G + 2 * w.g;
+    const size_t base = j * cg.outer + k0;
+    const double qy = a.x.vqy[j], qz0 = a.x.vqz[k0], qz1 = a.x.vqz[k0 + 1];
+    const double s0 = qy * qy + qz0 * qz0, s1 = qy * qy + qz1 * qz1;
+    // this tile's state, and the next tile's N, on their way while N is transformed
+    const int r = threadIdx.x % C::THREADS;
+    if (!a.from_spec) {
+      const size_t c0 = base - 2 * w.g;
+      prefetch_tile<C, N, G>(a.psiq + c0, opaque(cg.stride), r);
+      if (quasi) prefetch_tile<C, N, G>(a.psiq_old + c0, opaque(cg.stride), r);
+      if (!first) prefetch_tile<C, N, G>(a.Nq_old + c0, opaque(cg.stride), r);
+    }
+    if (const int nt = tile + gridDim.x * x_sets<N>(); nt < tiles && !a.from_spec)
+      prefetch_tile<C, N, G>(a.in + (nt / cg.kt) * cg.outer + (nt % cg.kt) * 2 * G, opaque(cg.stride), r);
+    if (!a.from_spec) {
+      Cx<T> u[F::E];
+      IO::load_pos(a.in + base, cg.stride, l, u, false);
+      F::forward(w, u, sh.xt, sh.tt);
+      IO::store_spec(a.Nq + base, cg.stride, l, u, false);
+      const int stride = opaque(cg.stride);
+#pragma unroll
+      for (int t = 0; t < F::E; ++t) {
+        const int k = l + F::L * t;
+        const size_t at = base + unsigned(k * stride);
+        const Cx<double> pq = ld2(a.psiq + at);
+        const Cx<double> po = quasi ? ld2(a.psiq_old + at) : Cx<double>{0.0, 0.0};
+        const Cx<T> no = first ? u[t] : ld2(a.Nq_old + at);   // quasi.cpp:1936-1938
+        auto advance = [&](double s, T n, T n_old, double p, double p_old) {
+          const double d = q02 - (sh.q[k] * sh.q[k] + s);
+          const double alin = a.ep - a.alpha * (d * d);
+          const double forcing = dsc * (3.0 * double(n) - double(n_old));
+          if (quasi) {
+            const double c1 = 2.0 - a.dt * a.rho_m * alin, c2 = 1.5 - a.dt * a.rho_m * alin;   // quasi.cpp:886-887
+            return (c1 * p - 0.5 * p_old + forcing) / c2;
+          }
+          const double c1 = 1.0 + dtd2 * alin, c2 = 1.0 - dtd2 * alin;   // quasi-stb.cpp:855-856
+          return (c1 * p + forcing) / c2;
+        };
+        const Cx<double> v{advance(s0, u[t].x, no.x, pq.x, po.x), advance(s1, u[t].y, no.y, pq.y, po.y)};
+        st2(a.psiq_new + at, v);
+        sh.spec[k * G + w.g] = v;
+      }
+    } else {
+      const int stride = opaque(cg.stride);
+#pragma unroll
+      for (int t = 0; t < FD::E; ++t) {
+        const int k = l + FD::L * t;
+        sh.spec[k * G + w.g] = ld2(a.psiq_new + base + unsigned(k * stride));
+      }
+    }
+    w.sync();
+#pragma unroll 1
+    for (int o = 0; o < 2; ++o) {   // psi, d_x psi
+      Cx<double> v[FD::E];
+#pragma unroll
+      for (int t = 0; t < FD::E; ++t) {
+        const int n = IOD::place(l + FD::L * t, o == 1);
+        v[t] = sh.spec[n * G + w.g];
+        if (o == 1) v[t] = cscale(v[t], -sh.q[n]);
+      }
+      FD::inverse(w, v, sh.xd, sh.td);
+      IOD::store_pos((o ? a.out1 : a.out0) + base, cg.stride, l, v, o == 1);
+    }
+    // the T fields: the multiplier of quasi.cpp:1044-1047, 1120-1186 (or
+    // quasi-stb.cpp:1019) in double, rounded once; grad lap psi is |q|^2 q_A psi^
+    // in each mode, the derivative -q_A of lap psi = -|q|^2 psi.  All of them are
+    //   (a0 + a1 q2) (b2 q2 + bx x + bc) + c,  q2 = |q|^2, x = q_x,
+    // so one copy of the code serves every output (a branch per output made the
+    // kernel outgrow the instruction cache).
+    sh.narrow_spectrum(w);
+#pragma unroll 1
+    for (int o = 0; o < (quasi ? 5 : 1); ++o) {
+      const bool ring = o < 2, x_axis = o == 2;
+      const double a0 = ring ? a.alpha * q02 : 0.0, a1 = ring ? -a.alpha : 1.0;
+      const double b2 = !quasi || o == 1 ? -1.0 : 0.0, bx = x_axis ? 1.0 : 0.0;
+      const double bc0 = !quasi ? q02 : o == 0 ? 1.0 : o == 3 ? qy : o == 4 ? qz0 : 0.0;
+      const double bc1 = o == 4 ? qz1 : bc0, c = quasi ? 0.0 : -a.ep;
+      Cx<T> u[F::E];
+      const int n0 = x_axis ? N - l : l, dn = x_axis ? -F::L : F::L;
+#pragma unroll
+      for (int t = 0; t < F::E; ++t) {
+        const int n = t == 0 && l == 0 ? 0 : n0 + dn * t;   // (mode 0: x = 0)
+        const Cx<T> y = sh.spect()[n * G + w.g];
+        const double x = sh.q[n], xx = x * x, bxx = bx * x;
+        auto mul = [&](double s, double bc) {
+          const double q2 = xx + s;
+          return (a0 + a1 * q2) * (b2 * q2 + (bxx + bc)) + c;
+        };
+        u[t] = Cx<T>{y.x * T(mul(s0, bc0)), y.y * T(mul(s1, bc1))};
+      }
+      F::inverse(w, u, sh.xt, sh.tt);
+      IO::store_pos(a.out[o] + base, cg.stride, l, u, x_axis);
+    }
+    w.sync();   // the next tile rewrites the spectrum
+  }
+}
+
+// Pressure, staggered Stokes projection (quasi.cpp:1336-1884) between the x
+// passes of the stress (and divv) and those of p and v.  Four groups of threads,
+// one per field: each transforms its input and leaves its spectrum in its exchange
+// buffer; after a CTA barrier all threads share the modes (a, b, c), replacing the
+// four inputs by the four outputs
+//   p = scale (-(q . S) / q^2 [+ nu D in stb]),  v = scale / (nu q^2) (S - q (q . S) / q^2 + nu q D)
+// and after another each group transforms one of those back.
+template <typename T>
+struct ProjectX {
+  const T* in[4];   // Sx (x sine), Sy, Sz by mode; divv
+  T* out[4];        // p, vx, vy, vz by mode
+  XTables x;
+  double nu, scale;
+  int variant, n0;   // n0: planes per emulated MPI rank (quasi.cpp:1641-1690)
+};
+// Tiles: 8 pencils in float (at N = 256 two CTAs of 512 threads per SM, 226 us at
+// 256^3; one of 1024 on 32 lanes per pencil: 268 us), 4 in double for N >= 64 and
+// at N = 512.
+template <typename T, int N> constexpr int project_pencils() {
+  return N >= 512 || (sizeof(T) == 8 && N >= 64) ? 4 : 8;
+}
+template <typename T, int N, int G>
+constexpr size_t project_smem() {
+  return PencilFFT<T, N>::table_bytes() +
+         size_t(4) * ColTile<N, G>::XCH * sizeof(Cx<T>) + N * sizeof(T);
+}
+template <typename T, int N, int G> constexpr int project_cta() { return 4 * ColTile<N, G>::THREADS; }
+// CTAs per SM that the registers must allow: 1024 threads in float with 8
+// elements per lane, else 512
+template <typename T, int N, int G>
+constexpr int project_ctas() {
+  constexpr int want = sizeof(T) == 4 ? 1024 : 512, nt = project_cta<T, N, G>();
+  return want > nt ? want / nt : 1;
+}
+template <typename T, int N, int G>
+__global__ void __launch_bounds__(project_cta<T, N, G>(), project_ctas<T, N, G>())
+    project_x_kernel(const __grid_constant__ ProjectX<T> a, Geom geom, int tiles, Tables<T> tb) {
+  using C = ColTile<N, G>;
+  using F = PencilFFT<T, N>;
+  using IO = ColIO<T, N>;
+  constexpr int NT = project_cta<T, N, G>();
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int field = threadIdx.x / C::THREADS;
+  Cx<T>* buf = reinterpret_cast<Cx<T>*>(smem_raw + F::table_bytes());
+  Cx<T>* xb = buf + field * C::XCH;
+  T* q = reinterpret_cast<T*>(buf + 4 * C::XCH);
+  const typename F::Tab t = F::fill_tables(reinterpret_cast<Cx<T>*>(smem_raw), tb, threadIdx.x, NT);
+  for (int e = threadIdx.x; e < N; e += NT) q[e] = T(a.x.vqx[e]);
+  __syncthreads();
+  const C w(threadIdx.x % C::THREADS, 1 + field);
+  const int l = w.l();
+  // padded place of mode N - (l + L i)
+  auto phi_mirror = [](int l1, int i) {
+    if constexpr (F::L % F::R1 == 0) return F::phi_read(F::L - l1, F::E - 1 - i);
+    else return int(F::phi(N - l1 - F::L * i));
+  };
+  const bool stb = a.variant != 0;
+  const T scale = T(a.scale), nu = T(a.nu), inu = T(1.0 / a.nu);
+  const ColGeom cg = col_geom<0, G>(geom);
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int b = tile / cg.kt, c00 = (tile - b * cg.kt) * 2 * G;
+    const size_t base = b * cg.outer + c00 + 2 * w.g;
+    const T qy = T(a.x.vqy[b]);
+    if (const int nt = tile + gridDim.x; nt < tiles && (field < 3 || !stb))
+      prefetch_tile<C, N, G>(a.in[field] + (nt / cg.kt) * cg.outer + (nt % cg.kt) * 2 * G, opaque(cg.stride),
+                             threadIdx.x % C::THREADS);
+    Cx<T> v[F::E];
+    if (field < 3 || !stb) {
+      IO::load_pos(a.in[field] + base, cg.stride, l, v, field == 0);
+      F::forward(w, v, xb, t);
+      if (field) {
+#pragma unroll
+        for (int i = 0; i < F::E; ++i) xb[w.at(F::phi_read(l, i))] = v[i];
+      } else {   // by mode: element k is mode N - k, element 0 nothing
+#pragma unroll
+        for (int i = 0; i < F::E; ++i) {
+          const bool none = i == 0 && l == 0;
+          xb[w.at(none ? 0 : phi_mirror(l, i))] = none ? Cx<T>{T(0), T(0)} : v[i];
+        }
+      }
+    } else {   // quasi-stb never transforms divv: its spectrum stays 0
+#pragma unroll
+      for (int i = 0; i < F::E; ++i) xb[w.at(F::phi_read(l, i))] = Cx<T>{T(0), T(0)};
+    }
+    __syncthreads();
+    // every mode once: all four spectra in, p and v out, in place.  halo: plane
+    // "i - 1" of S_x as halo #4 delivers it to vy and vz (quasi.cpp:1649)
+    constexpr int ITER = (N * G + NT - 1) / NT, MS = NT / G;   // modes between a thread's
+    const int m0 = threadIdx.x / G, pg = threadIdx.x % G, c0 = c00 + 2 * pg;
+    const T qz0 = T(a.x.vqz[c0]), qz1 = T(a.x.vqz[c0 + 1]);
+    auto place = [&](int i) {   // of mode m0 + i MS
+      if constexpr (MS % C::R1 == 0) return (m0 + m0 / C::R1) * G + pg + i * (MS + MS / C::R1) * G;
+      else return int(unsigned(m0 + i * MS) + unsigned(m0 + i * MS) / unsigned(C::R1)) * G + pg;
+    };
+    Cx<T> halo[ITER];
+    if (a.n0 < N) {
+#pragma unroll
+      for (int i = 0; i < ITER; ++i) {
+        const int m = m0 + i * MS, m1 = m > 0 && m % a.n0 == 0 ? m - a.n0 + 1 : m;
+        if (N * G % NT == 0 || m < N) halo[i] = buf[F::phi(m1) * G + pg];
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < ITER; ++i) {
+      const int m = m0 + i * MS, at = place(i);
+      if (N * G % NT && m >= N) break;
+      const Cx<T> sx = buf[at], sy = buf[C::XCH + at], sz = buf[2 * C::XCH + at], dv = buf[3 * C::XCH + at];
+      const Cx<T> sh = a.n0 < N ? halo[i] : sx;
+      const T qx = q[m];
+      Cx<T> p, vx, vy, vz;
+      auto one = [&](T x, T xh, T y, T z, T d, T qz, int c, T& po, T& vxo, T& vyo, T& vzo) {
+        const T q2 = qx * qx + qy * qy + qz * qz;
+        const T inv = m + b + c ? rcp(q2) : T(0);
+        const T yz = qy * y + qz * z, dot = (qx * x + yz) * inv, doth = (qx * xh + yz) * inv, nd = nu * d;
+        const T cv = scale * inv * inu;
+        po = stb ? (m * b * c ? scale * (nd - dot) : T(0)) : -scale * dot;
+        // no mode 0 of a sine axis; vy, vz: zero on the last y and z planes of
+        // the reference's index (quasi.cpp:1683-1872)
+        vxo = m > 0 ? cv * (x - qx * dot + qx * nd) : T(0);
+        vyo = b > 0 && c < geom.nz - 1 ? cv * (y - qy * doth + qy * nd) : T(0);
+        vzo = c > 0 && b < geom.ny - 1 ? cv * (z - qz * doth + qz * nd) : T(0);
+      };
+      one(sx.x, sh.x, sy.x, sz.x, dv.x, qz0, c0, p.x, vx.x, vy.x, vz.x);
+      one(sx.y, sh.y, sy.y, sz.y, dv.y, qz1, c0 + 1, p.y, vx.y, vy.y, vz.y);
+      buf[at] = p;
+      buf[C::XCH + at] = vx;
+      buf[2 * C::XCH + at] = vy;
+      buf[3 * C::XCH + at] = vz;
+    }
+    __syncthreads();
+    const bool sine = field == 1;   // vx
+    if (!sine) {
+#pragma unroll
+      for (int i = 0; i < F::E; ++i) v[i] = xb[w.at(F::phi_read(l, i))];
+    } else {   // (mode 0 of vx is zero)
+#pragma unroll
+      for (int i = 0; i < F::E; ++i) v[i] = xb[w.at(i == 0 && l == 0 ? 0 : phi_mirror(l, i))];
+    }
+    w.sync();   // read before the exchanges of the inverse overwrite it
+    if (stb && field == 0) {   // quasi-stb's pressure is not transformed back
+      IO::store_spec(a.out[0] + base, cg.stride, l, v, false);
+    } else {
+      F::inverse(w, v, xb, t);
+      IO::store_pos(a.out[field] + base, cg.stride, l, v, sine);
+    }
+    w.sync();   // the next tile rewrites this group's buffer
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Launchers, instantiated per type in col_pass_f32.cu and col_pass_f64.cu.
+// ---------------------------------------------------------------------------
+// Passes of njobs fields along axis 0 or 1, all forward (REDFT10 / RODFT10, the
+// result times scale) or all inverse.  vq: the axis's wavenumbers (kColGrad,
+// kColBoth).  narrow: tiles of 4 pencils where that makes them one warp's.
+template <typename T>
+cudaError_t launch_col_batch(const Geom& g, int axis, bool forward, const ColJobs<T>& jobs, int njobs, Tables<T> tb,
+                             const double* vq, T scale, bool narrow, int sms, cudaStream_t s);
+template <typename T>
+cudaError_t launch_density_x(const Geom& g, const DensityX<T>& a, Tables<double> tb64, Tables<T> tb, int sms,
+                             cudaStream_t s);
+template <typename T>
+cudaError_t launch_update_x(const Geom& g, const UpdateX<T>& a, Tables<double> tb64, Tables<T> tb, int sms,
+                            cudaStream_t s);
+template <typename T>
+cudaError_t launch_project_x(const Geom& g, const ProjectX<T>& a, Tables<T> tb, int sms, cudaStream_t s);
+
+template <typename T, int N>
+cudaError_t launch_density_x_n(const Geom& g, const DensityX<T>& a, Tables<double> tb64, Tables<T> tb, int sms,
+                               cudaStream_t s) {
+  constexpr int G = x_pencils<N>(), NT = x_cta<N, G>(), SETS = x_sets<N>();
+  constexpr size_t smem = x_stage_smem<T, N, G>();
+  auto kern = density_x_kernel<T, N, G>;
+  static std::atomic<int> cache[kMaxDevices];
+  int per_sm = 1;
+  const cudaError_t e = resident_ctas(kern, NT, smem, cache, &per_sm);
+  if (e != cudaSuccess) return e;
+  const int tiles = col_tiles<0>(g, G);
+  kern<<<std::min(per_sm * sms, (tiles + SETS - 1) / SETS), NT, smem, s>>>(a, g, tiles, tb64, tb);
+  return cudaGetLastError();
+}
+template <typename T, int N>
+cudaError_t launch_update_x_n(const Geom& g, const UpdateX<T>& a, Tables<double> tb64, Tables<T> tb, int sms,
+                              cudaStream_t s) {
+  constexpr int G = x_pencils<N>(), NT = x_cta<N, G>(), SETS = x_sets<N>();
+  constexpr size_t smem = x_stage_smem<T, N, G>();
+  auto kern = update_x_kernel<T, N, G>;
+  static std::atomic<int> cache[kMaxDevices];
+  int per_sm = 1;
+  const cudaError_t e = resident_ctas(kern, NT, smem, cache, &per_sm);
+  if (e != cudaSuccess) return e;
+  const int tiles = col_tiles<0>(g, G);
+  kern<<<std::min(per_sm * sms, (tiles + SETS - 1) / SETS), NT, smem, s>>>(a, g, tiles, tb64, tb);
+  return cudaGetLastError();
+}
+template <typename T, int N>
+cudaError_t launch_project_x_n(const Geom& g, const ProjectX<T>& a, Tables<T> tb, int sms, cudaStream_t s) {
+  constexpr int G = project_pencils<T, N>(), NT = project_cta<T, N, G>();
+  constexpr size_t smem = project_smem<T, N, G>();
+  auto kern = project_x_kernel<T, N, G>;
+  static std::atomic<int> cache[kMaxDevices];
+  int per_sm = 1;
+  const cudaError_t e = resident_ctas(kern, NT, smem, cache, &per_sm);
+  if (e != cudaSuccess) return e;
+  const int tiles = col_tiles<0>(g, G);
+  kern<<<std::min(per_sm * sms, tiles), NT, smem, s>>>(a, g, tiles, tb);
+  return cudaGetLastError();
+}
+
+#define QUASI_COL_LENGTHS(n, call)           \
+  switch (n) {                               \
+    case 8: return call(8);                  \
+    case 16: return call(16);                \
+    case 32: return call(32);                \
+    case 64: return call(64);                \
+    case 96: return call(96);                \
+    case 128: return call(128);              \
+    case 192: return call(192);              \
+    case 256: return call(256);              \
+    case 512: return call(512);              \
+    default: return cudaErrorInvalidValue;   \
+  }
+#define QUASI_COL_BATCH(N) launch_col_batch_n<QT, N>(g, axis, forward, jobs, njobs, tb, vq, scale, narrow, sms, s)
+#define QUASI_DENSITY_X(N) launch_density_x_n<QT, N>(g, a, tb64, tb, sms, s)
+#define QUASI_UPDATE_X(N) launch_update_x_n<QT, N>(g, a, tb64, tb, sms, s)
+#define QUASI_PROJECT_X(N) launch_project_x_n<QT, N>(g, a, tb, sms, s)
+
+}  // namespace quasi

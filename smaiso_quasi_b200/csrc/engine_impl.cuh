@@ -3,7 +3,9 @@
 #pragma once
 #include <cstdint>
 #include <fstream>
+#include <map>
 #include <mutex>
+#include <tuple>
 
 #include "engine.cuh"
 
@@ -61,12 +63,12 @@ static __global__ void diag_final_kernel(const double* partial, int nblocks, dou
 template <typename T>
 class Engine : public EngineBase {
  public:
-  // fields of the storage type (+ the float copies of psiq and rhoq); then
-  // the double fields: psiq x 3, rhoq, rho, rho_old, psi x 2, grad psi x 3
-  // (+ the scratch of the double transforms in the FP32 form)
-  // FP32: + the float copies of psi^, rho^; FP64: + the second grad rho buffers
-  static constexpr int kFields = 22 + (kStateCopy<T> ? 2 : 3);
-  static constexpr int kDFields = 11 + (kStateCopy<T> ? 1 : 0);
+  // fields of the storage type: N^ x 2, divv^, S x 3, v x 3, divv, p, df, the
+  // spectra of df, lap and grad lap psi, base, grad, grad rho's spectra x 2 (two
+  // of them in the FP64 form); double fields: psiq x 3, rhoq, psi x 2, grad psi x 3,
+  // rho x 2, the density scratch (x 2 in the FP64 form)
+  static constexpr int kFields = 19 + (kStateCopy<T> ? 6 : 4);
+  static constexpr int kDFields = 11 + (kStateCopy<T> ? 1 : 2);
   static constexpr int kPhases = 6;   // lcm of the 3-buffer psiq and 2-buffer Nq rotations
 
   explicit Engine(const quasi_config& cfg) : cfg_(cfg) {}
@@ -77,14 +79,8 @@ class Engine : public EngineBase {
       if (ge) cudaGraphExecDestroy(ge);
     for (auto& gr : graph_)
       if (gr) cudaGraphDestroy(gr);
-    if (slab_) {
-      MapCache::get().forget(slab_, static_cast<char*>(slab_) + size_t(kFields) * n_ * sizeof(T));
-      cudaFree(slab_);
-    }
-    if (dslab_) {
-      MapCache::get().forget(dslab_, dslab_ + size_t(kDFields) * n_);
-      cudaFree(dslab_);
-    }
+    if (slab_) cudaFree(slab_);
+    if (dslab_) cudaFree(dslab_);
     for (auto& t : tw64_) t.release();
     if (tc_owned_) cudaFree(tc_owned_);
     if (tma_err_) cudaFree(tma_err_);
@@ -95,9 +91,6 @@ class Engine : public EngineBase {
     for (auto& t : tw_) t.release();
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
-    for (auto& e : fork_ev_)
-      if (e) cudaEventDestroy(e);
-    if (stream2_) cudaStreamDestroy(stream2_);
     if (stream_) cudaStreamDestroy(stream_);
   }
 
@@ -107,10 +100,6 @@ class Engine : public EngineBase {
     g_ = Geom{cfg_.nx, cfg_.ny, cfg_.nz};
     n_ = size_t(g_.nx) * g_.ny * g_.nz;
     if (!cuda_ok(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "stream")) return QUASI_ERR_CUDA;
-    // second capture stream and fork/join events of the step graphs
-    if (!cuda_ok(cudaStreamCreateWithFlags(&stream2_, cudaStreamNonBlocking), "stream")) return QUASI_ERR_CUDA;
-    for (auto& e : fork_ev_)
-      if (!cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event")) return QUASI_ERR_CUDA;
     if (!cuda_ok(cudaEventCreate(&ev0_), "event") || !cuda_ok(cudaEventCreate(&ev1_), "event")) return QUASI_ERR_CUDA;
     const size_t bytes = size_t(kFields) * n_ * sizeof(T), dbytes = size_t(kDFields) * n_ * sizeof(double);
     if (cudaMalloc(&slab_, bytes) != cudaSuccess || cudaMalloc(&dslab_, dbytes) != cudaSuccess) {
@@ -167,114 +156,50 @@ class Engine : public EngineBase {
     if (cfg_.autotune == 1) {
       const int rc = autotune();
       if (rc) return rc;
-    } else if (cfg_.autotune == 2) {   // every warp-tile candidate (tests of those kernels)
-      for (auto& a : tune_.xywarp) a[0] = a[1] = true;
     }
     return capture();
   }
 
-  // Time each tunable pass's candidate kernels on the scratch fields (zeros)
-  // and keep the fastest: the x and y passes as CTA or warp tiles, per type; in the
-  // BF16X3 form the plain x and y passes on the tensor cores or by FFT.  The
-  // two candidates are timed in alternation (5 rounds of 10 launches each, the
-  // best round of each counts), and the default stays unless the other is
-  // faster by more than 3%.  The choices are kept per (device, grid, form) for
-  // the handles created later in the process (an ensemble's members of one
-  // grid tune once).
+  // In the BF16X3 form, time the plain float y pass on the tensor cores and by FFT
+  // on a scratch field (zeros), in alternation (5 rounds of 10 launches each, the
+  // best round of each counts); the tensor cores stay unless the FFT is faster by
+  // more than 3%.  The other forms have one kernel per stage and nothing to choose.
+  // The choice is kept per (device, grid) for the handles created later.
   int autotune() {
+    tune_.measured = true;
+    if (!tc_on_) return QUASI_OK;
     static std::mutex mu;
-    static std::map<std::tuple<int, int, int, int, int>, Tuning> cache;
-    const auto key = std::make_tuple(cfg_.device, g_.nx, g_.ny, g_.nz, cfg_.precision);
+    static std::map<std::tuple<int, int, int, int>, bool> cache;
+    const auto key = std::make_tuple(cfg_.device, g_.nx, g_.ny, g_.nz);
     {
       std::lock_guard<std::mutex> lk(mu);
       auto it = cache.find(key);
       if (it != cache.end()) {
-        tune_ = it->second;
+        tune_.tc_y = it->second;
         return QUASI_OK;
       }
     }
-    // *ms < 0: the candidate does not cover this shape (the step uses the
-    // general kernel there), nothing to choose
-    auto time = [&](auto&& launch, float* ms) -> bool {
-      const cudaError_t e0 = launch();
-      if (e0 == cudaErrorNotSupported) {
-        *ms = -1;
-        return true;
+    float best[2] = {1e30f, 1e30f};
+    for (int round = 0; round < 5; ++round)
+      for (int v = 0; v < 2; ++v) {
+        tune_.tc_y = v == 1;
+        set_phase(0);
+        YBatch<T> b;
+        b.add(c_.Sx);
+        auto launch = [&] { return y_passes(c_, false, b, tb_.t[1], stream_); };
+        float ms = 0;
+        if (!cuda_ok(launch(), "autotune") || !cuda_ok(cudaEventRecord(ev0_, stream_), "event")) return QUASI_ERR_CUDA;
+        for (int r = 0; r < 10; ++r)
+          if (!cuda_ok(launch(), "autotune")) return QUASI_ERR_CUDA;
+        if (!cuda_ok(cudaEventRecord(ev1_, stream_), "event") || !cuda_ok(cudaEventSynchronize(ev1_), "sync") ||
+            !cuda_ok(cudaEventElapsedTime(&ms, ev0_, ev1_), "elapsed"))
+          return QUASI_ERR_CUDA;
+        best[v] = std::min(best[v], ms);
       }
-      if (!cuda_ok(e0, "autotune")) return false;
-      if (!cuda_ok(cudaEventRecord(ev0_, stream_), "event")) return false;
-      for (int r = 0; r < 10; ++r)
-        if (!cuda_ok(launch(), "autotune")) return false;
-      if (!cuda_ok(cudaEventRecord(ev1_, stream_), "event") || !cuda_ok(cudaEventSynchronize(ev1_), "sync"))
-        return false;
-      return cuda_ok(cudaEventElapsedTime(ms, ev0_, ev1_), "elapsed");
-    };
-    // best[v] over alternating rounds of the two settings applied by set(v)
-    auto race = [&](auto&& set, auto&& launch, float best[2]) -> bool {
-      best[0] = best[1] = 1e30f;
-      for (int round = 0; round < 5; ++round)
-        for (int v = 0; v < 2; ++v) {
-          set(v);
-          use_tma();
-          float ms = 0;
-          if (!time(launch, &ms)) return false;
-          if (ms < 0) {
-            best[0] = best[1] = -1;
-            return true;
-          }
-          best[v] = std::min(best[v], ms);
-        }
-      return true;
-    };
-    auto better = [](const float ms[2], bool dflt) {   // the chosen setting
-      if (ms[0] < 0 || ms[1] < 0) return dflt;
-      const float cur = ms[dflt ? 1 : 0], alt = ms[dflt ? 0 : 1];
-      return alt < 0.97f * cur ? !dflt : dflt;
-    };
-    Tuning best = tune_;
-    // storage type and (FP32 form) double
-    for (int d = 0; d < (kStateCopy<T> ? 2 : 1); ++d) {
-      const int slot = kStateCopy<T> ? d : 1;
-      float ms[2];
-      // x and y passes as CTA or warp tiles (the plain pass decides for all
-      // passes of that axis and type)
-      for (int a = 0; a < 2; ++a) {
-        auto xy = [&]() -> cudaError_t {
-          if (d == 0) {
-            if (a == 0) return launch_pass<T, 0>(g_, E01, tb_.t[0], LoadField<T>{g_, c_.tmp}, StoreField<T>{g_, c_.tmp}, stream_);
-            return launch_pass<T, 1>(g_, E01, tb_.t[1], LoadField<T>{g_, c_.tmp}, StoreField<T>{g_, c_.tmp}, stream_);
-          }
-          if (a == 0)
-            return launch_pass<double, 0>(g_, E01, tb64_.t[0], LoadField<double>{g_, c_.tmp64},
-                                          StoreField<double>{g_, c_.tmp64}, stream_);
-          return launch_pass<double, 1>(g_, E01, tb64_.t[1], LoadField<double>{g_, c_.tmp64},
-                                        StoreField<double>{g_, c_.tmp64}, stream_);
-        };
-        const int tc_keep = tune_.tc_axes;
-        tune_.tc_axes = 0;   // the FFT passes are what is tuned here
-        if (!race([&](int v) { tune_.xywarp[a][slot] = v == 1; }, xy, ms)) return QUASI_ERR_CUDA;
-        tune_.tc_axes = tc_keep;
-        best.xywarp[a][slot] = better(ms, false);
-        tune_ = best;
-      }
-    }
-    if (tc_on_) {   // x (bit 0) and y (bit 1) on the tensor cores or by FFT
-      int axes = 0;
-      for (int a = 0; a < 2; ++a) {
-        float ms[2];
-        auto p = [&]() -> cudaError_t {
-          if (a == 0) return launch_pass<T, 0>(g_, E01, tb_.t[0], LoadField<T>{g_, c_.tmp}, StoreField<T>{g_, c_.tmp}, stream_);
-          return launch_pass<T, 1>(g_, E01, tb_.t[1], LoadField<T>{g_, c_.tmp}, StoreField<T>{g_, c_.tmp}, stream_);
-        };
-        if (!race([&](int v) { tune_.tc_axes = v ? (1 << a) : 0; }, p, ms)) return QUASI_ERR_CUDA;
-        if (better(ms, true)) axes |= 1 << a;
-      }
-      best.tc_axes = axes;
-    }
-    best.measured = true;
-    tune_ = best;
+    tune_.tc_y = !(best[0] < 0.97f * best[1]);
+    set_phase(0);
     std::lock_guard<std::mutex> lk(mu);
-    cache.emplace(key, best);
+    cache.emplace(key, tune_.tc_y);
     return QUASI_OK;
   }
 
@@ -306,8 +231,7 @@ class Engine : public EngineBase {
   int init() override {
     if (!have_psi_) { err = "quasi_init before quasi_set_psi"; return QUASI_ERR_STATE; }
     set_phase(0);
-    use_tma();
-    if (!cuda_ok(enqueue_init<T>(c_, tb_, tb64_, nloop_dev_, stream_), "init")) return QUASI_ERR_CUDA;
+    if (!cuda_ok(enqueue_init<T>(c_, tb_, tb64_, stream_), "init")) return QUASI_ERR_CUDA;
     if (!cuda_ok(cudaStreamSynchronize(stream_), "init sync")) return QUASI_ERR_CUDA;
     nloop_ = 0;
     initialized_ = true;
@@ -331,6 +255,7 @@ class Engine : public EngineBase {
 
   int synchronize() override {
     if (!cuda_ok(cudaStreamSynchronize(stream_), "step sync")) return QUASI_ERR_CUDA;
+    if (!c_.tc) return QUASI_OK;   // only the tensor-core passes wait on anything
     int tma_failed = 0;
     if (!cuda_ok(cudaMemcpy(&tma_failed, tma_err_, sizeof(int), cudaMemcpyDeviceToHost), "flag")) return QUASI_ERR_CUDA;
     if (tma_failed) {
@@ -403,7 +328,11 @@ class Engine : public EngineBase {
     set_phase(nloop_);
     uint64_t sum = kCheckSeed;
     for (const Field& fd : carried()) {
-      if (!cuda_ok(cudaMemcpy(host_stage_, fd.p, n_ * fd.elem, cudaMemcpyDeviceToHost), "D2H")) return QUASI_ERR_CUDA;
+      const void* p = fd.p;
+      if (fd.derive >= 0 && !cuda_ok(derived(fd.derive, &p), "derived field")) return QUASI_ERR_CUDA;
+      if (!cuda_ok(cudaMemcpyAsync(host_stage_, p, n_ * fd.elem, cudaMemcpyDeviceToHost, stream_), "D2H") ||
+          !cuda_ok(cudaStreamSynchronize(stream_), "sync"))
+        return QUASI_ERR_CUDA;
       sum = checksum(sum, host_stage_, n_ * fd.elem);
       f.write(static_cast<const char*>(host_stage_), n_ * fd.elem);
     }
@@ -444,12 +373,16 @@ class Engine : public EngineBase {
     for (const Field& fd : fields) {
       f.read(static_cast<char*>(host_stage_), std::streamsize(n_ * fd.elem));
       if (!f) { err = "checkpoint read failed"; return QUASI_ERR_IO; }
+      if (fd.derive >= 0) continue;   // follows from the state below
       if (!cuda_ok(cudaMemcpy(const_cast<void*>(fd.p), host_stage_, n_ * fd.elem, cudaMemcpyHostToDevice), "H2D"))
         return QUASI_ERR_CUDA;
     }
     set_phase(hd.nloop);
     int nl = int(hd.nloop);
     if (!cuda_ok(cudaMemcpy(nloop_dev_, &nl, sizeof(int), cudaMemcpyHostToDevice), "H2D")) return QUASI_ERR_CUDA;
+    if (!cuda_ok(enqueue_resume<T>(c_, tb_, tb64_, stream_), "resume") ||
+        !cuda_ok(cudaStreamSynchronize(stream_), "sync"))
+      return QUASI_ERR_CUDA;
     nloop_ = hd.nloop;
     have_psi_ = initialized_ = true;
     return QUASI_OK;
@@ -462,9 +395,9 @@ class Engine : public EngineBase {
   void note_steps(int n) override { nloop_ += n; }
   bool initialized() const override { return initialized_; }
   void tuning(int out[4]) const override {
-    for (int d = 0; d < 2; ++d)   // z passes always run as warp tiles (row_pass.cuh)
-      out[d] = 1 | (int(tune_.xywarp[0][d]) << 1) | (int(tune_.xywarp[1][d]) << 2);
-    out[2] = tc_on_ ? tune_.tc_axes : 0;
+    // z passes always run as warp tiles (row_pass.cuh), x / y passes with autotune = 2
+    for (int d = 0; d < 2; ++d) out[d] = 1 | (cfg_.autotune == 2 ? 6 : 0);
+    out[2] = tc_on_ && tune_.tc_y ? 2 : 0;
     out[3] = tune_.measured;
   }
 
@@ -480,14 +413,14 @@ class Engine : public EngineBase {
 
   int time_axis_pass(int axis, int reps, double* avg_ms) override {
     if (axis < 0 || axis > 2 || reps < 1) { err = "axis must be 0..2 and reps >= 1"; return QUASI_ERR_INVALID; }
-    T* d = c_.tmp;
-    use_tma();
+    T* d = c_.base;   // written and read within a step only
     auto one = [&]() -> cudaError_t {
-      if (axis == 0) return launch_pass<T, 0>(g_, E01, tb_.t[0], LoadField<T>{g_, d}, StoreField<T>{g_, d}, stream_);
-      if (axis == 1) return launch_pass<T, 1>(g_, E01, tb_.t[1], LoadField<T>{g_, d}, StoreField<T>{g_, d}, stream_);
-      const cudaError_t e = launch_zpass<T>(g_, E01, tb_.t[2], d, d, stream_);
-      if (e != cudaErrorNotSupported) return e;
-      return launch_pass<T, 2>(g_, E01, tb_.t[2], LoadField<T>{g_, d}, StoreField<T>{g_, d}, stream_);
+      if (axis == 1) {   // as a step's y pass runs (the tensor cores in the BF16X3 form)
+        YBatch<T> b;
+        b.add(d);
+        return y_passes(c_, false, b, tb_.t[1], stream_);
+      }
+      return plain_pass<T>(c_, axis, false, d, tb_.t[axis], stream_);
     };
     if (!cuda_ok(one(), "pass")) return QUASI_ERR_CUDA;   // warm
     if (!cuda_ok(cudaEventRecord(ev0_, stream_), "event")) return QUASI_ERR_CUDA;
@@ -546,23 +479,39 @@ class Engine : public EngineBase {
   struct Field {
     const void* p;
     size_t elem;
+    int derive = -1;   // >= 0: made from the state when saved, skipped when loaded
   };
-  // the state a step reads (at the phase set by set_phase(nloop))
+  // A checkpoint's fields (at the phase set by set_phase(nloop)).  Some are no
+  // longer stored as such between steps; the file keeps its layout.
   std::vector<Field> carried() {
     const size_t t = sizeof(T), d = sizeof(double);
-    std::vector<Field> v = {{c_.psiq, d}, {c_.psiq_old, d}, {c_.Nq_old, t}, {c_.rhoq, d},  {c_.rho_old, d},
+    std::vector<Field> v = {{c_.psiq, d}, {c_.psiq_old, d}, {c_.Nq_old, t}, {c_.rhoq, d},  {c_.rho, d},
                             {c_.rho, d},  {c_.vx, t},       {c_.vy, t},     {c_.vz, t},    {c_.divv, t},
                             {c_.divvq, t}, {c_.psi, d},     {c_.psi_old, d}, {c_.p, t},    {c_.df, t},
                             {c_.gx, d},    {c_.gy, d},      {c_.gz, d}};
-    if constexpr (kStateCopy<T>) {
-      v.push_back({c_.psiq_t, t});
-      v.push_back({c_.rhoq_t, t});
-    } else {   // grad rho, computed by the previous step
-      v.push_back({c_.rdx, t});
-      v.push_back({c_.rdy, t});
-      v.push_back({c_.rdz, t});
+    if constexpr (kStateCopy<T>) {   // the float copies of psi^ and rho^
+      v.push_back({nullptr, t, 0});
+      v.push_back({nullptr, t, 1});
+    } else {   // grad rho of rho^
+      for (int a = 0; a < 3; ++a) v.push_back({nullptr, t, a});
     }
     return v;
+  }
+  // A derived field of a checkpoint, in a buffer that a step writes before it
+  // reads it.
+  cudaError_t derived(int which, const void** p) {
+    T* out = c_.base;
+    *p = out;
+    if constexpr (kStateCopy<T>) {
+      to_storage_kernel<T><<<592, 256, 0, stream_>>>(which ? c_.rhoq : c_.psiq, out, n_);
+      return cudaGetLastError();
+    } else {
+      if (cfg_.variant != QUASI_VARIANT_QUASI) return cudaMemsetAsync(out, 0, n_ * sizeof(T), stream_);
+      if (which == 2)   // -vs_z[k] row[k + 1] of rho's spectrum
+        return launch_row_pass<T>(g_, O01, tb_.t[2], c_.law_next, out, 2, c_.vsz, sms_, true, stream_);
+      return launch_row_pass<T>(g_, E01, tb_.t[2], which ? c_.rdy : c_.rdx, out, 0, static_cast<const T*>(nullptr),
+                                sms_, true, stream_);
+    }
   }
   std::vector<Field> carried_at(long s) {
     const long keep = nloop_;
@@ -577,40 +526,26 @@ class Engine : public EngineBase {
   // Nq (computed this step) = B[s%2], Nq_old = B[(s+1)%2];
   // psi = C[s%2], psi_old = psi_new = C[(s+1)%2] (psi_old is read only by the
   // diagnostics after the step, when it is C[s%2] again);
-  // FP64 form: grad rho read = R[s%2], grad rho for the next step = R[(s+1)%2].
+  // rho = D[s%2], the step's new rho D[(s+1)%2]; grad rho's spectra alike;
+  // law = E[(s+1)%2], law_next = E[s%2] (one buffer in the FP32 form).
   void set_phase(long s) {
     c_.psiq = psiq_buf_[s % 3];
     c_.psiq_old = psiq_buf_[(s + 2) % 3];
     c_.psiq_new = psiq_buf_[(s + 1) % 3];
-    if constexpr (!kStateCopy<T>) {   // the FP64 form reads the state itself
-      c_.psiq_t = reinterpret_cast<T*>(c_.psiq);
-      c_.rhoq_t = reinterpret_cast<T*>(c_.rhoq);
-    }
     c_.Nq = nq_buf_[s % 2];
     c_.Nq_old = nq_buf_[(s + 1) % 2];
     c_.psi = psi_buf_[s % 2];
     c_.psi_old = psi_buf_[(s + 1) % 2];
     c_.psi_new = psi_buf_[(s + 1) % 2];
-    // grad rho (the FP32 form has one buffer and no next)
-    T* const* rd = rd_buf_[kStateCopy<T> ? 0 : s % 2];
+    c_.rho = rho_buf_[s % 2];
+    c_.rho_new = rho_buf_[(s + 1) % 2];
+    c_.law = law_buf_[(s + 1) % 2];
+    c_.law_next = law_buf_[s % 2];
+    T* const* rd = rd_buf_[s % 2];
+    T* const* rn = rd_buf_[(s + 1) % 2];
     c_.rdx = rd[0]; c_.rdy = rd[1]; c_.rdz = rd[2];
-    if constexpr (!kStateCopy<T>) {
-      T* const* rn = rd_buf_[(s + 1) % 2];
-      c_.rdnx = rn[0]; c_.rdny = rn[1]; c_.rdnz = rn[2];
-    } else {
-      c_.rdnx = c_.rdny = c_.rdnz = nullptr;
-    }
-  }
-
-  void use_tma() {
-    TmaConfig& t = tma_config();
-    t.err = tma_err_;
-    t.sms = sms_;
-    t.enabled = true;
-    t.tc = tc_on_ ? &tc_tables_ : nullptr;
-    t.tc_axes = tune_.tc_axes;
-    for (int a = 0; a < 2; ++a)
-      for (int d = 0; d < 2; ++d) t.xywarp[a][d] = tune_.xywarp[a][d];
+    c_.rdx_new = rn[0]; c_.rdy_new = rn[1]; c_.rdz_new = rn[2];
+    c_.tc = tc_on_ && tune_.tc_y ? &tc_tables_ : nullptr;
   }
 
   bool cuda_ok(cudaError_t e, const char* what) {
@@ -624,13 +559,15 @@ class Engine : public EngineBase {
     auto next = [&]() { T* p = f; f += n_; return p; };
     c_.g = g_;
     const double* t = tabs_;
-    c_.vqx = t;                 c_.vsx = t + g_.nx;
-    c_.vqy = t + 2 * g_.nx;     c_.vsy = c_.vqy + g_.ny;
-    c_.vqz = t + 2 * g_.nx + 2 * g_.ny; c_.vsz = c_.vqz + g_.nz;
+    // per axis: vq (mode i at i), vs (mode i + 1 at i); then the filter per axis
+    c_.x.vqx = t;
+    c_.x.vqy = c_.vqy = t + 2 * g_.nx;
+    c_.x.vqz = c_.vqz = t + 2 * g_.nx + 2 * g_.ny;
+    c_.vsz = c_.vqz + g_.nz;
     const double* ft = t + 2 * (g_.nx + g_.ny + g_.nz);
-    c_.fx = ft;
-    c_.fy = ft + g_.nx;
-    c_.fz = ft + g_.nx + g_.ny;
+    c_.x.fx = ft;
+    c_.x.fy = ft + g_.nx;
+    c_.x.fz = ft + g_.nx + g_.ny;
     (void)h;
     const bool quasi = cfg_.variant == QUASI_VARIANT_QUASI;
     c_.ep = -0.001 * cfg_.ep_arg;                                   // quasi.cpp:187
@@ -645,29 +582,28 @@ class Engine : public EngineBase {
     c_.divv_switch = cfg_.divv_switch;
     c_.n0 = g_.nx / (cfg_.emulate_ranks > 0 ? cfg_.emulate_ranks : 1);
     c_.nloop = nloop_dev_;
-    c_.store_dtpsi = quasi ? 0 : 1;
+    c_.sms = sms_;
+    c_.narrow = cfg_.autotune == 2;
+    c_.err = tma_err_;
     double* dfp = dslab_;
     auto dnext = [&]() { double* p = dfp; dfp += n_; return p; };
     for (auto& b : psiq_buf_) b = dnext();
     c_.rhoq = dnext();
-    c_.rho = dnext(); c_.rho_old = dnext();
     for (auto& b : psi_buf_) b = dnext();
     c_.gx = dnext(); c_.gy = dnext(); c_.gz = dnext();
+    for (auto& b : rho_buf_) b = dnext();
+    law_buf_[0] = dnext();
+    law_buf_[1] = kStateCopy<T> ? law_buf_[0] : dnext();
     for (auto& b : nq_buf_) b = next();
-    if constexpr (kStateCopy<T>) {
-      c_.psiq_t = next();
-      c_.rhoq_t = next();
-    }
     c_.divvq = next(); c_.Sx = next(); c_.Sy = next(); c_.Sz = next();
     c_.vx = next(); c_.vy = next(); c_.vz = next(); c_.divv = next(); c_.p = next();
-    c_.df = next(); c_.lap = next();
-    for (auto& b : rd_buf_[0]) b = next();
-    if constexpr (!kStateCopy<T>)
-      for (auto& b : rd_buf_[1]) b = next();
+    c_.df = next(); c_.dfs = next(); c_.lap = next();
     c_.ldx = next(); c_.ldy = next(); c_.ldz = next();
-    c_.sh = next(); c_.dtpsi = next(); c_.tmp = next();
-    if constexpr (kStateCopy<T>) c_.tmp64 = dnext();
-    else c_.tmp64 = reinterpret_cast<double*>(c_.tmp);
+    c_.base = next(); c_.grad = next();
+    c_.mu = c_.lap;       // quasi-stb: mu replaces sh's spectrum row by row
+    c_.dtpsi = c_.ldx;    // and has no grad lap psi
+    for (auto& set : rd_buf_)
+      for (int a = 0; a < (kStateCopy<T> ? 3 : 2); ++a) set[a] = next();
     set_phase(0);
     // every field inside its slab (the counts above are the slabs' sizes)
     layout_ok_ = f == static_cast<T*>(slab_) + size_t(kFields) * n_ && dfp == dslab_ + size_t(kDFields) * n_;
@@ -703,10 +639,9 @@ class Engine : public EngineBase {
   int capture_phase(int ph) {
     cudaGraph_t graph = nullptr;
     set_phase(ph);
-    use_tma();
     if (!cuda_ok(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "begin capture"))
       return QUASI_ERR_CUDA;
-    cudaError_t e = enqueue_step<T>(c_, tb_, tb64_, nloop_dev_, stream_, stream2_, fork_ev_);
+    cudaError_t e = enqueue_step<T>(c_, tb_, tb64_, stream_);
     cudaError_t e2 = cudaStreamEndCapture(stream_, &graph);
     if (!cuda_ok(e, "enqueue step") || !cuda_ok(e2, "end capture")) {
       if (graph) cudaGraphDestroy(graph);
@@ -741,16 +676,13 @@ class Engine : public EngineBase {
   bool tc_on_ = false;
   // the autotuner's choices (see autotune())
   struct Tuning {
-    bool xywarp[2][2] = {{false, false}, {false, false}};   // [axis x, y][float, double]
-    int tc_axes = 3;
+    bool tc_y = true;
     bool measured = false;
   } tune_;
   bool layout_ok_ = false;
   double* tabs_ = nullptr;
   int* nloop_dev_ = nullptr;
   double* partial_ = nullptr;
-  cudaStream_t stream2_ = nullptr;
-  cudaEvent_t fork_ev_[12] = {};
   int* tma_err_ = nullptr;
   int sms_ = 148;
   void* host_stage_ = nullptr;
@@ -764,7 +696,9 @@ class Engine : public EngineBase {
   double* psiq_buf_[3] = {};
   T* nq_buf_[2] = {};
   double* psi_buf_[2] = {};
-  T* rd_buf_[2][3] = {};   // grad rho (x, y, z); the second set in the FP64 form only
+  double* rho_buf_[2] = {};
+  double* law_buf_[2] = {};
+  T* rd_buf_[2][3] = {};   // grad rho's spectra
   int graph_kernels_ = 0;
   long nloop_ = 0;
 };

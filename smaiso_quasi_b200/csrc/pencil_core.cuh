@@ -17,8 +17,8 @@
 // are those of r2r_core.cuh.
 //
 // `W` places a pencil's lanes: l(), partner() (the lane of the warp that holds
-// l' = (L - l) mod L of the same pencil), at(e) (element e of this pencil in the
-// exchange buffer), shfl(value, lane) and sync() (all lanes of the exchange
+// l' = (L - l) mod L of the same pencil), at(place) (a padded place of this pencil
+// in the exchange buffer), shfl(value, lane) and sync() (all lanes of the exchange
 // buffer).  A test runs the same code with host threads as lanes.
 #pragma once
 #include "r2r_core.cuh"
@@ -53,11 +53,17 @@ template <typename T> struct Dft<T, 12> {
 };
 
 // Lanes per pencil and radices: the first radix is E = N / L, and every stage's
-// N / R butterflies are a multiple of L.
+// N / R butterflies are a multiple of L.  The plain plans have the fewest
+// exchanges (a float row pass at N = 256: 23 us with 16 lanes, 29 with 32).  The
+// wide ones have half the elements per lane, for double stages that would have
+// too few warps otherwise (a double row pass: 48.5 us and 49.5, the second at
+// half the registers and exchange buffer per warp).
 struct RowPlan {
   int lanes, n_stages, r[3];
 };
-QHD constexpr RowPlan row_plan(int n) {
+QHD constexpr RowPlan row_plan(int n, bool wide = false) {
+  if (wide && n == 256) return {32, 3, {8, 8, 4}};
+  if (wide && n == 128) return {16, 3, {8, 4, 4}};
   switch (n) {
     case 8: return {4, 3, {2, 2, 2}};
     case 16: return {4, 2, {4, 4, 0}};
@@ -72,29 +78,51 @@ QHD constexpr RowPlan row_plan(int n) {
   }
 }
 
-template <typename T, int N>
+template <typename T, int N, bool WIDE = false>
 struct PencilFFT {
-  static constexpr RowPlan plan = row_plan(N);
+  static constexpr RowPlan plan = row_plan(N, WIDE);
   static_assert(plan.lanes > 0, "unsupported transform length");
   static constexpr int L = plan.lanes, E = N / L, H = E / 2;
   static constexpr int R1 = plan.r[0];
   static_assert(R1 == E && E % 2 == 0, "the first radix is a lane's share");
-  // padded place of element e: the first stage writes with stride R1
+  // Padded place of element e of the exchange buffer, e + e / R1 (the first stage
+  // writes with stride R1).  In the forms the stages use, as a lane's base plus a
+  // constant, which the accesses take as immediates:
   QHD static constexpr int phi(int e) { return e + e / R1; }
   static constexpr int kPadded = N - 1 + (N - 1) / R1 + 1;
-  // tables in shared memory, per CTA: the first stage's twiddles W_N^{l u} as
-  // [u][l], the quarter-wave table, and W_N^t when there is a third stage
-  static constexpr int kTables = plan.n_stages > 2 ? 3 : 2;
+  // element l + L t
+  QHD static int phi_read(int l, int t) {
+    if constexpr (L % R1 == 0) return l + l / R1 + t * (L + L / R1);
+    else if constexpr (R1 % L == 0) return l + (L * t + L * t / R1);
+    else return int(unsigned(l + L * t) + unsigned(l + L * t) / unsigned(R1));
+  }
+  // output u of butterfly b = l + L c of stage ST (radix R, stride s)
+  template <int ST>
+  QHD static int phi_write(int l, int c, int u) {
+    if constexpr (ST == 0) {
+      return (R1 + 1) * l + (R1 + 1) * L * c + u;
+    } else {   // s = R1: e = q + R1 (R2 p + u), p = b / R1, q = b % R1
+      constexpr int R = plan.r[1];
+      if constexpr (L % R1 == 0) return l % R1 + (R1 + 1) * R * (l / R1) + (R1 + 1) * (R * (L / R1) * c + u);
+      const unsigned b = unsigned(l + L * c), p = b / unsigned(R1);
+      return int(b - p * R1 + (R1 + 1) * R * p) + (R1 + 1) * u;
+    }
+  }
+  // Tables in shared memory, per CTA: the first stage's twiddles W_N^{l u} as
+  // [u][l], i times the quarter-wave table, and the second stage's W_N^{s p u} (s = R1)
+  // as [u][p] when there is a third.
+  static constexpr int R2 = plan.r[1], P2 = N / (R1 * R2);
+  static constexpr int kTables = 2 * N + (plan.n_stages > 2 ? R2 * P2 : 0);   // complex entries
   struct Tab {
-    const Cx<T>*tw1, *quarter, *root;
+    const Cx<T>*tw1, *iquarter, *tw2;
   };
-  static constexpr size_t table_bytes() { return size_t(kTables) * N * sizeof(Cx<T>); }
-  // fills the tables at `t` (kTables * N entries); the caller synchronises
+  static constexpr size_t table_bytes() { return (size_t(kTables) * sizeof(Cx<T>) + 15) / 16 * 16; }
+  // fills the tables at `t`; the caller synchronises
   QHD static Tab fill_tables(Cx<T>* t, Tables<T> tb, int tid, int nt) {
     for (int e = tid; e < N; e += nt) {
       t[e] = tb.root[(e / L) * (e % L)];
-      t[N + e] = tb.quarter[e];
-      if (kTables > 2) t[2 * N + e] = tb.root[e];
+      t[N + e] = Cx<T>{-tb.quarter[e].y, tb.quarter[e].x};
+      if (plan.n_stages > 2 && e < R2 * P2) t[2 * N + e] = tb.root[R1 * (e / P2) * (e % P2)];
     }
     return Tab{t, t + N, t + 2 * N};
   }
@@ -116,19 +144,37 @@ struct PencilFFT {
 #pragma unroll
         for (int u = 0; u < R; ++u) v[c + B * u] = a[u];
       } else {
-        const int b = l + L * c, p = b / s, q = b - p * s;
+        const int p = ST == 0 ? 0 : int(unsigned(l + L * c) / unsigned(s));
 #pragma unroll
         for (int u = 0; u < R; ++u) {
           Cx<T> f = a[u];
-          if (u) f = cmul(f, ST == 0 ? tb.tw1[u * L + l] : tb.root[s * p * u]);
-          xb[w.at(q + s * (R * p + u))] = f;
+          if (u) f = cmul(f, ST == 0 ? tb.tw1[u * L + l] : tb.tw2[u * P2 + p]);
+          if constexpr (W::template split<T>()) v[c + B * u] = f;
+          else xb[w.at(phi_write<ST>(l, c, u))] = f;
         }
       }
     }
-    if constexpr (!last) {
+    if constexpr (!last && W::template split<T>()) {   // the real parts, then the imaginary ones
+      T* xr = reinterpret_cast<T*>(xb);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int c = 0; c < B; ++c)
+#pragma unroll
+          for (int u = 0; u < R; ++u) xr[w.at(phi_write<ST>(l, c, u))] = h ? v[c + B * u].y : v[c + B * u].x;
+        w.sync();
+#pragma unroll
+        for (int t = 0; t < E; ++t) {
+          const T x = xr[w.at(phi_read(l, t))];
+          if (h) v[t].y = x;
+          else v[t].x = x;
+        }
+        w.sync();
+      }
+    } else if constexpr (!last) {
       w.sync();
 #pragma unroll
-      for (int t = 0; t < E; ++t) v[t] = xb[w.at(l + L * t)];
+      for (int t = 0; t < E; ++t) v[t] = xb[w.at(phi_read(l, t))];
       w.sync();
     }
   }
@@ -140,8 +186,9 @@ struct PencilFFT {
   }
 
   // Inverse kinds (REDFT01; RODFT01 with its input reversed by the caller):
-  // v[t] = (y_k of row a, y_k of row b) -> F_k, the complex DFT whose conjugate
-  // holds the permuted outputs.  v_k = quarter_k ((a_k + b_{N-k}) + i (a_{N-k} - b_k)).
+  // v[t] = (y_k of row a, y_k of row b) -> v[t] = (b, a) of the permuted outputs.
+  // The inverse DFT of z is the forward DFT with real and imaginary parts swapped
+  // on both sides; the swapped input is i quarter_k ((a_k + b_{N-k}) + i (a_{N-k} - b_k)).
   template <class W>
   QHD static void inverse(const W& w, Cx<T>* v, Cx<T>* xb, const Tab& tb) {
     const int l = w.l(), src = w.partner();
@@ -152,8 +199,8 @@ struct PencilFFT {
       const Cx<T> lo = v[t], hi = v[u], up = v[t + 1];
       const Cx<T> plo = w.shfl(l ? hi : prev, src), phi_ = w.shfl(l ? lo : up, src);
       prev = hi;
-      v[t] = cmul(tb.quarter[l + L * t], Cx<T>{lo.x + plo.y, plo.x - lo.y});
-      v[u] = cmul(tb.quarter[l + L * u], Cx<T>{hi.x + phi_.y, phi_.x - hi.y});
+      v[t] = cmul(tb.iquarter[l + L * t], Cx<T>{lo.x + plo.y, plo.x - lo.y});
+      v[u] = cmul(tb.iquarter[l + L * u], Cx<T>{hi.x + phi_.y, phi_.x - hi.y});
     }
     dft(w, v, xb, tb);
   }
@@ -172,13 +219,13 @@ struct PencilFFT {
       const Cx<T> lo = v[t], hi = v[u], up = v[t + 1];
       const Cx<T> plo = w.shfl(l ? hi : prev, src), phi_ = w.shfl(l ? lo : up, src);
       prev = hi;
-      v[t] = unpack(lo, plo, tb.quarter[l + L * t]);
-      v[u] = unpack(hi, phi_, tb.quarter[l + L * u]);
+      v[t] = unpack(lo, plo, tb.iquarter[l + L * t]);
+      v[u] = unpack(hi, phi_, tb.iquarter[l + L * u]);
     }
   }
-  // y_k of both rows from Z_k and Z_{N-k}
+  // y_k of both rows from Z_k and Z_{N-k}; q = i quarter_k
   QHD static Cx<T> unpack(Cx<T> z, Cx<T> n, Cx<T> q) {
-    return Cx<T>{q.x * (z.x + n.x) - q.y * (z.y - n.y), q.x * (z.y + n.y) + q.y * (z.x - n.x)};
+    return Cx<T>{q.y * (z.x + n.x) + q.x * (z.y - n.y), q.y * (z.y + n.y) - q.x * (z.x - n.x)};
   }
 
   // Position of y_k along the axis.  sine: the kind's own order (k reversed);
@@ -195,26 +242,32 @@ struct PencilFFT {
 // adjacent positions (n, n + 1), n = 2 l + 2 L t, is this lane's element t and
 // lane L - 1 - l's element E - 1 - t: one shuffle gives each lane adjacent pairs
 // of both rows, and every real-space access is a 2-element vector.
-template <typename T, int N>
-struct RowFFT : PencilFFT<T, N> {
-  using P = PencilFFT<T, N>;
+template <typename T, int N, bool WIDE = false>
+struct RowFFT : PencilFFT<T, N, WIDE> {
+  using P = PencilFFT<T, N, WIDE>;
   using P::E;
   using P::H;
   using P::L;
   static constexpr int PPW = 32 / L, ROWS = 2 * PPW;   // pencils and rows of a warp
-  // complex elements between the pencils of a warp: the lanes of one access
-  // phase (16 in float, 8 in double) that span several pencils hit distinct banks
+  // Double rows of more than 8 elements per lane exchange real and imaginary
+  // parts one after the other: half the buffer at the same time (48.5 us at
+  // N = 256 either way; in float 23 -> 27 us).
+  static constexpr bool kSplit = sizeof(T) == 8 && E > 8;
+  // elements between the pencils of a warp: the lanes of one access phase (16 of
+  // 8 bytes, 8 of 16) that span several pencils hit distinct banks
   static constexpr int pencil_stride() {
-    constexpr int ph = sizeof(T) == 8 ? 8 : 16;
+    constexpr int ph = sizeof(T) == 8 && !kSplit ? 8 : 16;
     int x = P::kPadded;
     if (L < ph)
       while (x % ph != L) ++x;
     return x;
   }
   static constexpr int XS = pencil_stride();
-  static constexpr int XCH = PPW * XS;   // complex elements of a warp's exchange buffer
-  // F_k -> adjacent positions: a[t] = row a at (n, n + 1), b[t] = row b, n = 2 l + 2 L t.
-  // In place: v[t] = row a's pair, v[E - 1 - t] = row b's.  sine: odd positions negated.
+  static constexpr size_t xch_bytes() {   // of a warp's exchange buffer
+    return (size_t(PPW) * XS * (kSplit ? sizeof(T) : sizeof(Cx<T>)) + 15) / 16 * 16;
+  }
+  // Permuted outputs (b, a) -> adjacent positions: v[t] = row a at (n, n + 1), v[E - 1 - t]
+  // = row b, n = 2 l + 2 L t.  sine: odd positions negated.
   template <class W>
   QHD static void to_pairs(const W& w, Cx<T>* v, bool sine) {
     const int src = w.mirror();
@@ -222,11 +275,11 @@ struct RowFFT : PencilFFT<T, N> {
 #pragma unroll
     for (int t = 0; t < H; ++t) {
       const Cx<T> o = w.shfl(v[E - 1 - t], src), e = v[t];
-      v[t] = Cx<T>{e.x, s * o.x};
-      v[E - 1 - t] = Cx<T>{-e.y, -s * o.y};
+      v[t] = Cx<T>{e.y, s * o.y};
+      v[E - 1 - t] = Cx<T>{e.x, s * o.x};
     }
   }
-  // the reverse, for a forward kind's input
+  // pairs -> (a, b) of the permuted positions, a forward kind's input
   template <class W>
   QHD static void from_pairs(const W& w, Cx<T>* v, bool sine) {
     const int src = w.mirror();
@@ -243,15 +296,16 @@ struct RowFFT : PencilFFT<T, N> {
 
 #ifdef __CUDACC__
 // The lanes of a warp as RowFFT places them.
-template <typename T, int N>
+template <typename T, int N, bool WIDE = false>
 struct RowWarp {
-  using F = RowFFT<T, N>;
+  using F = RowFFT<T, N, WIDE>;
+  template <typename> static constexpr bool split() { return F::kSplit; }
   int lane;
   __device__ __forceinline__ int l() const { return lane % F::L; }
   __device__ __forceinline__ int pencil() const { return lane / F::L; }
   __device__ __forceinline__ int partner() const { return lane - l() + ((F::L - l()) & (F::L - 1)); }
   __device__ __forceinline__ int mirror() const { return lane + F::L - 1 - 2 * l(); }
-  __device__ __forceinline__ int at(int e) const { return pencil() * F::XS + F::phi(e); }
+  __device__ __forceinline__ int at(int place) const { return pencil() * F::XS + place; }
   __device__ __forceinline__ void sync() const { __syncwarp(); }
   __device__ __forceinline__ Cx<T> shfl(Cx<T> v, int src) const {
     return Cx<T>{__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)};
@@ -265,9 +319,11 @@ struct RowWarp {
 // Neighbouring l differ in parity, which puts a half-warp's float accesses to
 // the exchange rows [e][g] on distinct banks.  Tiles of one warp synchronise the
 // warp, wider ones a named barrier.
-template <int N, int G>
+template <int N, int G, bool WIDE = false, bool SPLIT = false>
 struct ColTile {
-  static constexpr int L = row_plan(N).lanes, R1 = N / L, S = 32 / G;
+  // double real and imaginary parts exchanged one after the other
+  template <typename T> static constexpr bool split() { return SPLIT && sizeof(T) == 8; }
+  static constexpr int L = row_plan(N, WIDE).lanes, R1 = N / L, S = 32 / G;
   static constexpr int THREADS = G * L;
   static_assert(THREADS % 32 == 0 && S >= 2, "a tile is whole warps");
   static constexpr int ROWS = N - 1 + (N - 1) / R1 + 1;   // padded rows of G of the exchange buffer
@@ -282,7 +338,7 @@ struct ColTile {
   }
   __device__ __forceinline__ int l() const { return ll; }
   __device__ __forceinline__ int partner() const { return part; }
-  __device__ __forceinline__ int at(int e) const { return (e + e / R1) * G + g; }
+  __device__ __forceinline__ int at(int place) const { return place * G + g; }
   __device__ __forceinline__ void sync() const {
     if constexpr (THREADS == 32) __syncwarp();
     else asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(THREADS) : "memory");

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "engine.cuh"
+#include "r2r_pass.cuh"
 
 namespace quasi {
 
@@ -77,8 +78,8 @@ struct R2R : R2RBase {
     const Geom g{nx, ny, nz};
     cudaError_t e;
     use_tma();
-    const int k3[3] = {kind[0], kind[1], kind[2]};
-    e = yz3(g, tb, k3, d, StoreField<T>{g, d}, s);
+    e = launch_row_pass<T>(g, kind[2], tb.t[2], d, d, 0, static_cast<const T*>(nullptr), sms, true, s);
+    if (e == cudaSuccess) e = launch_pass<T, 1>(g, kind[1], tb.t[1], LoadField<T>{g, d}, StoreField<T>{g, d}, s);
     if (e == cudaSuccess) e = launch_pass<T, 0>(g, kind[0], tb.t[0], LoadField<T>{g, d}, StoreField<T>{g, d}, s);
     end_tma();
     return e;

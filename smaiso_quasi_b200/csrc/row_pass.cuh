@@ -41,6 +41,11 @@ __device__ __forceinline__ void st2(T* p, Cx<T> v) {
   *reinterpret_cast<typename Vec2<T>::type*>(p) = w;
 }
 
+// Starts fetching `bytes` (a multiple of 16) at p (16-byte aligned) into L2.
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // Resident CTAs per SM of a kernel, its dynamic shared memory allowed; found
 // once per device and instantiation.
 constexpr int kMaxDevices = 64;
@@ -110,7 +115,7 @@ struct RowIO {
 constexpr int kRowWarps = 8;   // warps per CTA of the row kernels
 template <typename T, int N>
 constexpr size_t row_smem(int warps = kRowWarps) {
-  return RowFFT<T, N>::table_bytes() + size_t(warps) * RowFFT<T, N>::XCH * sizeof(Cx<T>);
+  return RowFFT<T, N>::table_bytes() + size_t(warps) * RowFFT<T, N>::xch_bytes();
 }
 
 // Groups are walked from the last x plane to the first when rev: the pass before
@@ -125,10 +130,9 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2)
   constexpr bool fwd = KIND == E10 || KIND == O10, sine = KIND == O10 || KIND == O01;
   constexpr bool prefetch = sizeof(T) == 4 && KS != 2;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  Cx<T>* tab = reinterpret_cast<Cx<T>*>(smem_raw);
   const int warp = threadIdx.x >> 5;
-  Cx<T>* xb = tab + F::kTables * N + warp * F::XCH;
-  const typename F::Tab t = F::fill_tables(tab, tb, threadIdx.x, 32 * kRowWarps);
+  Cx<T>* xb = reinterpret_cast<Cx<T>*>(smem_raw + F::table_bytes() + warp * F::xch_bytes());
+  const typename F::Tab t = F::fill_tables(reinterpret_cast<Cx<T>*>(smem_raw), tb, threadIdx.x, 32 * kRowWarps);
   __syncthreads();
   const RowWarp<T, N> w{int(threadIdx.x & 31)};
   const int l = w.l(), stride = gridDim.x * kRowWarps;
