@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include "row_pass.cuh"
+#include "tma.cuh"
 
 namespace quasi {
 
@@ -34,19 +35,15 @@ __device__ __forceinline__ int opaque(int x) {
   return x;
 }
 
-// The tile's columns in a field along one axis: element (n, this lane's pair).
+// The tiles of an x stage in a field.
 struct ColGeom {
-  int stride;      // elements between rows along the axis
-  int kt;          // tiles per outer index
-  size_t outer;    // elements between outer indices
+  int stride;      // elements between rows along x
+  int kt;          // tiles per j
+  size_t outer;    // elements between j
 };
-template <int AXIS, int G>
-__host__ __device__ __forceinline__ ColGeom col_geom(const Geom& g) {
-  if (AXIS == 1) return {g.nz, g.nz / (2 * G), size_t(g.ny) * g.nz};
-  return {g.ny * g.nz, g.nz / (2 * G), size_t(g.nz)};
-}
-template <int AXIS>
-inline int col_tiles(const Geom& g, int G) { return (AXIS == 1 ? g.nx : g.ny) * (g.nz / (2 * G)); }
+template <int G>
+__device__ __forceinline__ ColGeom x_geom(const Geom& g) { return {g.ny * g.nz, g.nz / (2 * G), size_t(g.nz)}; }
+inline int x_tiles(const Geom& g, int G) { return g.ny * (g.nz / (2 * G)); }
 
 // The threads of a tile start fetching its N rows of 2 G elements into L2.
 template <class C, int N, int G, typename T>
@@ -118,7 +115,8 @@ enum ColOp : int {
   kColCos = 0,    // cosine kind
   kColSine = 1,   // sine kind, its spectrum by mode number
   kColGrad = 2,   // (inverse) cosine spectrum c_m -> RODFT01 of the modes -q_m c_m: the derivative along the axis
-  kColBoth = 3    // (inverse) dst = the cosine transform, dst2 = the derivative, one tile load each
+  kColBoth = 3,   // (inverse) dst = the cosine transform, dst2 = the derivative, one tile load
+  kColIndex = 4   // sine kind, its spectrum in FFTW's order (mode m at m - 1)
 };
 template <typename T>
 struct ColJob {
@@ -131,91 +129,216 @@ template <typename T>
 struct ColJobs {
   ColJob<T> job[kMaxJobs];
 };
+struct ColMaps {   // a job's fields as tensor maps (the tile's box)
+  CUtensorMap src[kMaxJobs], dst[kMaxJobs], dst2[kMaxJobs];
+  int op[kMaxJobs];
+};
+// Waits of the passes: the flag that a timed-out wait sets, its limit in polls, and
+// (failure tests) a tile whose copy is never issued.
+constexpr uint32_t kPollLimit = 1u << 24;
+struct ColWait {
+  int* err = nullptr;
+  uint32_t polls = kPollLimit;
+  int skip = -1;
+};
 
 // Pencils of a tile (G): 8, as nz is a multiple of 16; 4 as "warp tiles", which
 // make tiles of the lengths with 8 lanes one warp's own (no barrier).
 // threads of a CTA: at least four warps, one tile per THREADS
 template <int N, int G> constexpr int col_cta() { return ColTile<N, G>::THREADS >= 128 ? ColTile<N, G>::THREADS : 128; }
 
+// Shared memory of a pass: per tile the landing buffers and the exchange buffer
+// (also the staging rows of the tile's store), then tables and barriers.
 template <typename T, int N, int G>
-constexpr size_t col_batch_smem() {
-  return PencilFFT<T, N>::table_bytes() + N * sizeof(T) +
-         size_t(col_cta<N, G>() / ColTile<N, G>::THREADS) * ColTile<N, G>::XCH * sizeof(Cx<T>);
-}
-template <typename T, int N, int G, bool FWD>
-__global__ void __launch_bounds__(col_cta<N, G>(), 512 / col_cta<N, G>())
-    col_batch_kernel(const __grid_constant__ ColJobs<T> jobs, int njobs, ColGeom cg, int tiles, Tables<T> tb,
-                     const double* vq, T scale) {
+struct ColSmem {
   using C = ColTile<N, G>;
+  static constexpr int NT = col_cta<N, G>(), SETS = NT / C::THREADS;
+  // tiles in flight beyond the one worked on: a register's worth of time is enough
+  // for float (22.7 us a pass at 256^3 with one or two buffers), double takes two
+  // (51 -> 48 us)
+  static constexpr int BUFS = sizeof(T) == 8 ? 2 : 1;
+  static constexpr int TILE = 2 * G * N;   // elements
+  static constexpr size_t xch_bytes() { return (size_t(C::XCH) * sizeof(Cx<T>) + 127) / 128 * 128; }
+  static constexpr size_t set_bytes() { return size_t(BUFS) * TILE * sizeof(T) + xch_bytes(); }
+  static constexpr size_t bytes() {
+    return SETS * set_bytes() + PencilFFT<T, N>::table_bytes() + N * sizeof(T) + SETS * BUFS * sizeof(uint64_t);
+  }
+  static_assert(TILE * sizeof(T) <= size_t(C::XCH) * sizeof(Cx<T>), "the staging rows overlay the exchange buffer");
+  static_assert(TILE * sizeof(T) % 128 == 0, "tensor copies land on 128-byte boundaries");
+};
+
+// Tiles arrive by TMA, land as rows [n][2G] and are read into registers once; the
+// next tile's copy is issued as soon as every thread has read.  The output rows are
+// staged over the exchange buffer and leave by a TMA store.  Bound: HBM; with the
+// threads loading and storing global rows themselves the address arithmetic took a
+// third of the instructions (float 28.6 us a pass at 256^3, 22.7 now; double 50 -> 48).
+template <typename T, int N, int G, bool FWD>
+__global__ void __launch_bounds__(col_cta<N, G>(), (sizeof(T) == 8 ? 384 : 512) / col_cta<N, G>())
+    col_batch_kernel(const __grid_constant__ ColMaps maps, int axis, int kt, int tiles, int njobs, Tables<T> tb,
+                     const double* vq, T scale, ColWait wait) {
+  using S = ColSmem<T, N, G>;
+  using C = typename S::C;
   using F = PencilFFT<T, N>;
-  using IO = ColIO<T, N>;
-  constexpr int NT = col_cta<N, G>(), SETS = NT / C::THREADS;
+  constexpr int SETS = S::SETS, BUFS = S::BUFS, P = 2 * G, SUB = (N + 255) / 256, BN = N / SUB;   // box sides <= 256
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  const int set = threadIdx.x / C::THREADS;
-  Cx<T>* xb = reinterpret_cast<Cx<T>*>(smem_raw + F::table_bytes()) + set * C::XCH;
-  T* q = reinterpret_cast<T*>(reinterpret_cast<Cx<T>*>(smem_raw + F::table_bytes()) + SETS * C::XCH);
-  const typename F::Tab t = F::fill_tables(reinterpret_cast<Cx<T>*>(smem_raw), tb, threadIdx.x, NT);
-  for (int e = threadIdx.x; e < N; e += NT) q[e] = vq ? T(-vq[e]) : T(0);
+  const int set = threadIdx.x / C::THREADS, r = threadIdx.x % C::THREADS;
+  T* raw = reinterpret_cast<T*>(smem_raw + set * S::set_bytes());
+  Cx<T>* xb = reinterpret_cast<Cx<T>*>(raw + BUFS * S::TILE);
+  T* stage = reinterpret_cast<T*>(xb);
+  unsigned char* sm = smem_raw + SETS * S::set_bytes();
+  const typename F::Tab t = F::fill_tables(reinterpret_cast<Cx<T>*>(sm), tb, threadIdx.x, S::NT);
+  sm += F::table_bytes();
+  T* q = reinterpret_cast<T*>(sm);
+  for (int e = threadIdx.x; e < N; e += S::NT) q[e] = vq ? T(-vq[e]) : T(0);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + N * sizeof(T)) + set * BUFS;
+  if (r == 0) {
+#pragma unroll
+    for (int b = 0; b < BUFS; ++b) mbar_init(&bar[b], 1);
+    mbar_fence_init();
+    const int j = min(int(blockIdx.x * SETS + set) / tiles, njobs - 1);
+    prefetch_map(&maps.src[j]);
+    prefetch_map(&maps.dst[j]);
+  }
   __syncthreads();
-  const C w(threadIdx.x % C::THREADS, 1 + set);
-  const int l = w.l();
-  for (int x = blockIdx.x * SETS + set; x < tiles * njobs; x += gridDim.x * SETS) {
-    const int j = x / tiles, tile = x - j * tiles;
-    const ColJob<T>& jb = jobs.job[j];
-    auto corner = [&](int i) { return (i / cg.kt) * cg.outer + (i % cg.kt) * 2 * G; };
-    const size_t base = corner(tile) + 2 * w.g;
-    Cx<T> v[F::E];
-    if constexpr (FWD) {
-      const bool sine = jb.op == kColSine;
-      IO::load_pos(jb.src + base, cg.stride, l, v, sine);
-      F::forward(w, v, xb, t);
-      if (scale != T(1)) {
+  pdl_begin();
+  const C w(r, 1 + set);
+  const int l = w.l(), all = tiles * njobs, stride = gridDim.x * SETS;
+  auto issue = [&](int x, int b) {
+    if (x == wait.skip) return;
+    const int j = x / tiles, tile = x - j * tiles, o = tile / kt, k0 = (tile - o * kt) * P;
+    mbar_expect_tx(&bar[b], S::TILE * sizeof(T));
 #pragma unroll
-        for (int i = 0; i < F::E; ++i) v[i] = cscale(v[i], scale);
-      }
-      IO::store_spec(jb.dst + base, cg.stride, l, v, sine);
-    } else {
-      // kColBoth: the derivative first; the tile is read again (from L1 / L2)
-      // before the cosine transform may overwrite it
+    for (int sb = 0; sb < SUB; ++sb)
+      tma_load_3d(raw + b * S::TILE + sb * BN * P, &maps.src[j], &bar[b], k0, axis == 1 ? sb * BN : o,
+                  axis == 1 ? o : sb * BN);
+  };
+  int x = blockIdx.x * SETS + set;
+  if (r == 0) {
+#pragma unroll
+    for (int b = 0; b < BUFS; ++b)
+      if (x + b * stride < all) issue(x + b * stride, b);
+  }
+  for (int it = 0; x < all; x += stride, ++it) {
+    const int b = it % BUFS, j = x / tiles, tile = x - j * tiles, op = maps.op[j];
+    const T* tl = raw + b * S::TILE + 2 * w.g;
+    bool ok = mbar_wait_bounded(&bar[b], (it / BUFS) & 1, wait.polls);
+    // kColBoth: the derivative first
 #pragma unroll 1
-      for (int pass = jb.op == kColBoth ? 0 : 1; pass < 2; ++pass) {
-        const bool grad = pass == 0 || jb.op == kColGrad, sine = grad || jb.op == kColSine;
-        IO::load_spec(jb.src + base, cg.stride, l, v, sine);
-        if (grad) {
+    for (int pass = !FWD && op == kColBoth ? 0 : 1; pass < 2; ++pass) {
+      const bool grad = !FWD && (pass == 0 || op == kColGrad), sine = grad || op == kColSine || op == kColIndex;
+      const int order = sine && op != kColIndex ? N - l : N - 1 - l;   // place of a sine spectrum's element l
+      Cx<T> v[F::E];
+      if constexpr (FWD) {
+        const T s = sine ? T(-1) : T(1);
 #pragma unroll
-          for (int i = 0; i < F::E; ++i) v[i] = cscale(v[i], q[IO::place(l + F::L * i, true)]);
+        for (int i = 0; i < F::E; ++i) {
+          v[i] = ld2(tl + F::pos(l + F::L * i) * P);
+          if (i >= F::H) v[i] = cscale(v[i], s);
         }
+      } else if (!sine) {
+#pragma unroll
+        for (int i = 0; i < F::E; ++i) v[i] = ld2(tl + (l + F::L * i) * P);
+      } else {
+#pragma unroll
+        for (int i = 0; i < F::E; ++i) {
+          const int n = i == 0 && order == N ? 0 : order - F::L * i;
+          v[i] = ld2(tl + n * P);
+          if (grad) v[i] = cscale(v[i], q[n]);
+          if (i == 0 && order == N) v[i] = Cx<T>{T(0), T(0)};   // the top mode has no place
+        }
+      }
+      if (r == 0) bulk_wait_read0();   // the previous store has read the staging rows
+      ok = w.sync_all(ok);
+      if (!ok) break;
+      if (pass == 1 && r == 0 && x + BUFS * stride < all) {   // this landing buffer has been read
+        fence_proxy_async_smem();
+        issue(x + BUFS * stride, b);
+      }
+      if constexpr (FWD) {
+        F::forward(w, v, xb, t);
+        if (scale != T(1)) {
+#pragma unroll
+          for (int i = 0; i < F::E; ++i) v[i] = cscale(v[i], scale);
+        }
+        if (!sine) {
+#pragma unroll
+          for (int i = 0; i < F::E; ++i) st2(stage + 2 * w.g + (l + F::L * i) * P, v[i]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < F::E; ++i) {
+            const bool none = i == 0 && order == N;
+            st2(stage + 2 * w.g + (none ? 0 : order - F::L * i) * P, none ? Cx<T>{T(0), T(0)} : v[i]);
+          }
+        }
+      } else {
         F::inverse(w, v, xb, t);
-        IO::store_pos((pass == 0 ? jb.dst2 : jb.dst) + base, cg.stride, l, v, sine);
+        const T s = sine ? T(-1) : T(1);
+#pragma unroll
+        for (int i = 0; i < F::E; ++i) {
+          const Cx<T> u = i < F::H ? v[i] : cscale(v[i], s);
+          st2(stage + 2 * w.g + F::pos(l + F::L * i) * P, Cx<T>{u.y, u.x});
+        }
+      }
+      fence_proxy_async_smem();
+      w.sync();
+      if (r == 0) {
+        const int o = tile / kt, k0 = (tile - o * kt) * P;
+#pragma unroll
+        for (int sb = 0; sb < SUB; ++sb)
+          tma_store_3d(pass == 0 ? &maps.dst2[j] : &maps.dst[j], stage + sb * BN * P, k0, axis == 1 ? sb * BN : o,
+                       axis == 1 ? o : sb * BN);
+        bulk_commit();
       }
     }
+    if (!ok) {   // a copy never arrived: flag it, wait for the others in flight, leave
+      if (r == 0) {
+        atomicExch(wait.err, 1);
+        for (int d = 1; d < BUFS; ++d) {
+          const int xo = x + d * stride;
+          if (xo < all && xo != wait.skip) mbar_wait_bounded(&bar[(it + d) % BUFS], ((it + d) / BUFS) & 1, wait.polls);
+        }
+      }
+      break;
+    }
   }
+  if (r == 0) bulk_wait0();
 }
 
 template <typename T, int N, int G, bool FWD>
 cudaError_t launch_col_batch_g(const Geom& g, int axis, const ColJobs<T>& jobs, int njobs, Tables<T> tb,
-                               const double* vq, T scale, int sms, cudaStream_t s) {
-  constexpr int NT = col_cta<N, G>(), SETS = NT / ColTile<N, G>::THREADS;
+                               const double* vq, T scale, const ColWait& wait, int sms, cudaStream_t s) {
+  using S = ColSmem<T, N, G>;
   auto kern = col_batch_kernel<T, N, G, FWD>;
   static std::atomic<int> cache[kMaxDevices];
   int per_sm = 1;
-  const cudaError_t e = resident_ctas(kern, NT, col_batch_smem<T, N, G>(), cache, &per_sm);
+  const cudaError_t e = resident_ctas(kern, S::NT, S::bytes(), cache, &per_sm);
   if (e != cudaSuccess) return e;
-  const int tiles = axis == 1 ? col_tiles<1>(g, G) : col_tiles<0>(g, G), work = (tiles * njobs + SETS - 1) / SETS;
-  kern<<<std::min(per_sm * sms, work), NT, col_batch_smem<T, N, G>(), s>>>(
-      jobs, njobs, axis == 1 ? col_geom<1, G>(g) : col_geom<0, G>(g), tiles, tb, vq, scale);
-  return cudaGetLastError();
+  constexpr uint32_t BN = N > 256 ? N / ((N + 255) / 256) : N;
+  const uint32_t box[3] = {uint32_t(2 * G), axis == 1 ? BN : 1, axis == 1 ? 1 : BN};
+  ColMaps maps{};
+  for (int j = 0; j < njobs; ++j) {
+    const ColJob<T>& jb = jobs.job[j];
+    maps.op[j] = jb.op;
+    if (!make_field_map(&maps.src[j], jb.src, int(sizeof(T)), g.nx, g.ny, g.nz, box)) return cudaErrorInvalidValue;
+    if (jb.dst == jb.src) maps.dst[j] = maps.src[j];
+    else if (!make_field_map(&maps.dst[j], jb.dst, int(sizeof(T)), g.nx, g.ny, g.nz, box)) return cudaErrorInvalidValue;
+    if (jb.dst2 && !make_field_map(&maps.dst2[j], jb.dst2, int(sizeof(T)), g.nx, g.ny, g.nz, box))
+      return cudaErrorInvalidValue;
+  }
+  const int kt = g.nz / (2 * G), tiles = (axis == 1 ? g.nx : g.ny) * kt, work = (tiles * njobs + S::SETS - 1) / S::SETS;
+  return launch_dependent(kern, std::min(per_sm * sms, work), S::NT, S::bytes(), s, maps, axis, kt, tiles, njobs, tb,
+                          vq, scale, wait);
 }
 template <typename T, int N>
 cudaError_t launch_col_batch_n(const Geom& g, int axis, bool forward, const ColJobs<T>& jobs, int njobs, Tables<T> tb,
-                               const double* vq, T scale, bool narrow, int sms, cudaStream_t s) {
+                               const double* vq, T scale, const ColWait& wait, bool narrow, int sms, cudaStream_t s) {
   if constexpr (row_plan(N).lanes == 8) {
     if (narrow)
-      return forward ? launch_col_batch_g<T, N, 4, true>(g, axis, jobs, njobs, tb, vq, scale, sms, s)
-                     : launch_col_batch_g<T, N, 4, false>(g, axis, jobs, njobs, tb, vq, scale, sms, s);
+      return forward ? launch_col_batch_g<T, N, 4, true>(g, axis, jobs, njobs, tb, vq, scale, wait, sms, s)
+                     : launch_col_batch_g<T, N, 4, false>(g, axis, jobs, njobs, tb, vq, scale, wait, sms, s);
   }
-  return forward ? launch_col_batch_g<T, N, 8, true>(g, axis, jobs, njobs, tb, vq, scale, sms, s)
-                 : launch_col_batch_g<T, N, 8, false>(g, axis, jobs, njobs, tb, vq, scale, sms, s);
+  return forward ? launch_col_batch_g<T, N, 8, true>(g, axis, jobs, njobs, tb, vq, scale, wait, sms, s)
+                 : launch_col_batch_g<T, N, 8, false>(g, axis, jobs, njobs, tb, vq, scale, wait, sms, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -320,6 +443,7 @@ struct XStage {
     xt = reinterpret_cast<Cx<T>*>(sm);
     spec = reinterpret_cast<Cx<double>*>(sm + x_xch_bytes<N, G>());
     __syncthreads();
+    pdl_begin();
   }
   // the tile's spectrum in T; FP32: the same bytes, after narrow_spectrum()
   __device__ __forceinline__ Cx<T>* spect() const { return reinterpret_cast<Cx<T>*>(spec); }
@@ -354,7 +478,7 @@ __global__ void __launch_bounds__(x_cta<N, G>(), x_ctas<N>())
   const X sh(smem_raw, set, tb64, tb, a.x.vqx, a.x.fx);
   const C w(threadIdx.x % C::THREADS, 1 + set);
   const int l = w.l();
-  const ColGeom cg = col_geom<0, G>(geom);
+  const ColGeom cg = x_geom<G>(geom);
   for (int tile = blockIdx.x * x_sets<N>() + set; tile < tiles; tile += gridDim.x * x_sets<N>()) {
     const int j = tile / cg.kt, k0 = (tile - j * cg.kt) * 2 * G + 2 * w.g;
     const size_t base = j * cg.outer + k0;
@@ -426,7 +550,7 @@ __global__ void __launch_bounds__(x_cta<N, G>(), x_ctas<N>())
   const C w(threadIdx.x % C::THREADS, 1 + set);
   const int l = w.l();
   const bool quasi = a.variant == 0, first = *a.nloop == 0;
-  const ColGeom cg = col_geom<0, G>(geom);
+  const ColGeom cg = x_geom<G>(geom);
   const double dtd2 = a.dt / 2, dsc = dtd2 * a.scale, q02 = a.q0 * a.q0;
   for (int tile = blockIdx.x * x_sets<N>() + set; tile < tiles; tile += gridDim.x * x_sets<N>()) {
     const int j = tile / cg.kt, k0 = (tile - j * cg.kt) * 2 * G + 2 * w.g;
@@ -575,6 +699,7 @@ __global__ void __launch_bounds__(project_cta<T, N, G>(), project_ctas<T, N, G>(
   const typename F::Tab t = F::fill_tables(reinterpret_cast<Cx<T>*>(smem_raw), tb, threadIdx.x, NT);
   for (int e = threadIdx.x; e < N; e += NT) q[e] = T(a.x.vqx[e]);
   __syncthreads();
+  pdl_begin();
   const C w(threadIdx.x % C::THREADS, 1 + field);
   const int l = w.l();
   // padded place of mode N - (l + L i)
@@ -584,7 +709,7 @@ __global__ void __launch_bounds__(project_cta<T, N, G>(), project_ctas<T, N, G>(
   };
   const bool stb = a.variant != 0;
   const T scale = T(a.scale), nu = T(a.nu), inu = T(1.0 / a.nu);
-  const ColGeom cg = col_geom<0, G>(geom);
+  const ColGeom cg = x_geom<G>(geom);
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int b = tile / cg.kt, c00 = (tile - b * cg.kt) * 2 * G;
     const size_t base = b * cg.outer + c00 + 2 * w.g;
@@ -684,7 +809,7 @@ __global__ void __launch_bounds__(project_cta<T, N, G>(), project_ctas<T, N, G>(
 // kColBoth).  narrow: tiles of 4 pencils where that makes them one warp's.
 template <typename T>
 cudaError_t launch_col_batch(const Geom& g, int axis, bool forward, const ColJobs<T>& jobs, int njobs, Tables<T> tb,
-                             const double* vq, T scale, bool narrow, int sms, cudaStream_t s);
+                             const double* vq, T scale, const ColWait& wait, bool narrow, int sms, cudaStream_t s);
 template <typename T>
 cudaError_t launch_density_x(const Geom& g, const DensityX<T>& a, Tables<double> tb64, Tables<T> tb, int sms,
                              cudaStream_t s);
@@ -704,9 +829,8 @@ cudaError_t launch_density_x_n(const Geom& g, const DensityX<T>& a, Tables<doubl
   int per_sm = 1;
   const cudaError_t e = resident_ctas(kern, NT, smem, cache, &per_sm);
   if (e != cudaSuccess) return e;
-  const int tiles = col_tiles<0>(g, G);
-  kern<<<std::min(per_sm * sms, (tiles + SETS - 1) / SETS), NT, smem, s>>>(a, g, tiles, tb64, tb);
-  return cudaGetLastError();
+  const int tiles = x_tiles(g, G);
+  return launch_dependent(kern, std::min(per_sm * sms, (tiles + SETS - 1) / SETS), NT, smem, s, a, g, tiles, tb64, tb);
 }
 template <typename T, int N>
 cudaError_t launch_update_x_n(const Geom& g, const UpdateX<T>& a, Tables<double> tb64, Tables<T> tb, int sms,
@@ -718,9 +842,8 @@ cudaError_t launch_update_x_n(const Geom& g, const UpdateX<T>& a, Tables<double>
   int per_sm = 1;
   const cudaError_t e = resident_ctas(kern, NT, smem, cache, &per_sm);
   if (e != cudaSuccess) return e;
-  const int tiles = col_tiles<0>(g, G);
-  kern<<<std::min(per_sm * sms, (tiles + SETS - 1) / SETS), NT, smem, s>>>(a, g, tiles, tb64, tb);
-  return cudaGetLastError();
+  const int tiles = x_tiles(g, G);
+  return launch_dependent(kern, std::min(per_sm * sms, (tiles + SETS - 1) / SETS), NT, smem, s, a, g, tiles, tb64, tb);
 }
 template <typename T, int N>
 cudaError_t launch_project_x_n(const Geom& g, const ProjectX<T>& a, Tables<T> tb, int sms, cudaStream_t s) {
@@ -731,9 +854,8 @@ cudaError_t launch_project_x_n(const Geom& g, const ProjectX<T>& a, Tables<T> tb
   int per_sm = 1;
   const cudaError_t e = resident_ctas(kern, NT, smem, cache, &per_sm);
   if (e != cudaSuccess) return e;
-  const int tiles = col_tiles<0>(g, G);
-  kern<<<std::min(per_sm * sms, tiles), NT, smem, s>>>(a, g, tiles, tb);
-  return cudaGetLastError();
+  const int tiles = x_tiles(g, G);
+  return launch_dependent(kern, std::min(per_sm * sms, tiles), NT, smem, s, a, g, tiles, tb);
 }
 
 #define QUASI_COL_LENGTHS(n, call)           \
@@ -749,7 +871,7 @@ cudaError_t launch_project_x_n(const Geom& g, const ProjectX<T>& a, Tables<T> tb
     case 512: return call(512);              \
     default: return cudaErrorInvalidValue;   \
   }
-#define QUASI_COL_BATCH(N) launch_col_batch_n<QT, N>(g, axis, forward, jobs, njobs, tb, vq, scale, narrow, sms, s)
+#define QUASI_COL_BATCH(N) launch_col_batch_n<QT, N>(g, axis, forward, jobs, njobs, tb, vq, scale, wait, narrow, sms, s)
 #define QUASI_DENSITY_X(N) launch_density_x_n<QT, N>(g, a, tb64, tb, sms, s)
 #define QUASI_UPDATE_X(N) launch_update_x_n<QT, N>(g, a, tb64, tb, sms, s)
 #define QUASI_PROJECT_X(N) launch_project_x_n<QT, N>(g, a, tb, sms, s)

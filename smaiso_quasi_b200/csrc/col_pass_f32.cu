@@ -6,7 +6,8 @@ using QT = float;
 
 template <>
 cudaError_t launch_col_batch<QT>(const Geom& g, int axis, bool forward, const ColJobs<QT>& jobs, int njobs,
-                                 Tables<QT> tb, const double* vq, QT scale, bool narrow, int sms, cudaStream_t s) {
+                                 Tables<QT> tb, const double* vq, QT scale, const ColWait& wait, bool narrow, int sms,
+                                 cudaStream_t s) {
   QUASI_COL_LENGTHS(axis == 1 ? g.ny : g.nx, QUASI_COL_BATCH)
 }
 template <>

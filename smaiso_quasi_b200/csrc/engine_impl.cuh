@@ -255,7 +255,6 @@ class Engine : public EngineBase {
 
   int synchronize() override {
     if (!cuda_ok(cudaStreamSynchronize(stream_), "step sync")) return QUASI_ERR_CUDA;
-    if (!c_.tc) return QUASI_OK;   // only the tensor-core passes wait on anything
     int tma_failed = 0;
     if (!cuda_ok(cudaMemcpy(&tma_failed, tma_err_, sizeof(int), cudaMemcpyDeviceToHost), "flag")) return QUASI_ERR_CUDA;
     if (tma_failed) {

@@ -343,6 +343,21 @@ struct ColTile {
     if constexpr (THREADS == 32) __syncwarp();
     else asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(THREADS) : "memory");
   }
+  // sync(), and whether `ok` held for every thread of the tile
+  __device__ __forceinline__ bool sync_all(bool ok) const {
+    if constexpr (THREADS == 32) {
+      return __all_sync(0xffffffffu, ok);
+    } else {
+      uint32_t r;
+      asm volatile(
+          "{\n .reg .pred p, q;\n setp.ne.u32 q, %3, 0;\n barrier.cta.red.and.pred p, %1, %2, q;\n"
+          " selp.u32 %0, 1, 0, p;\n}\n"
+          : "=r"(r)
+          : "r"(bar), "n"(THREADS), "r"(uint32_t(ok))
+          : "memory");
+      return r != 0;
+    }
+  }
   template <typename T>
   __device__ __forceinline__ Cx<T> shfl(Cx<T> v, int src) const {
     return Cx<T>{__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)};

@@ -7,7 +7,6 @@
 #include <vector>
 
 #include "engine.cuh"
-#include "r2r_pass.cuh"
 
 namespace quasi {
 
@@ -19,26 +18,10 @@ struct R2RBase {
   int* tma_err = nullptr;
   int sms = 148;
   int inject_skip = -1;             // fault injection for the next execution
-  uint32_t inject_polls = kTmaPollLimit;
+  uint32_t inject_polls = kPollLimit;
   tc::Tables4 tc_tables{};   // the tensor-core form's matrices (precision BF16X3_TC)
   void* tc_owned = nullptr;
   bool tc_on = false;
-  void use_tma() {
-    TmaConfig& t = tma_config();
-    t.err = tma_err;
-    t.sms = sms;
-    t.enabled = true;
-    t.skip_tile = inject_skip;
-    t.poll_limit = inject_polls;
-    t.tc = tc_on ? &tc_tables : nullptr;
-    t.tc_axes = 3;
-  }
-  void end_tma() {   // the injection lasts one execution
-    TmaConfig& t = tma_config();
-    t.tc = nullptr;
-    t.skip_tile = inject_skip = -1;
-    t.poll_limit = inject_polls = kTmaPollLimit;
-  }
   // after a synchronised execution: did a tile wait give up?
   cudaError_t timed_out(bool* out) {
     int f = 0;
@@ -73,15 +56,43 @@ struct R2R : R2RBase {
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return e;
     return cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
   }
+  // z, y, x pass in place.  The passes' tensor copies need 16-byte aligned data;
+  // other data goes through a buffer allocated in stream order.
   cudaError_t exec(void* data, cudaStream_t s) override {
-    T* d = static_cast<T*>(data);
-    const Geom g{nx, ny, nz};
+    const size_t bytes = size_t(nx) * ny * nz * sizeof(T);
+    void* d = data;
     cudaError_t e;
-    use_tma();
-    e = launch_row_pass<T>(g, kind[2], tb.t[2], d, d, 0, static_cast<const T*>(nullptr), sms, true, s);
-    if (e == cudaSuccess) e = launch_pass<T, 1>(g, kind[1], tb.t[1], LoadField<T>{g, d}, StoreField<T>{g, d}, s);
-    if (e == cudaSuccess) e = launch_pass<T, 0>(g, kind[0], tb.t[0], LoadField<T>{g, d}, StoreField<T>{g, d}, s);
-    end_tma();
+    if (reinterpret_cast<uintptr_t>(data) % 16) {
+      if ((e = cudaMallocAsync(&d, bytes, s)) != cudaSuccess) return e;
+      e = cudaMemcpyAsync(d, data, bytes, cudaMemcpyDeviceToDevice, s);
+    } else {
+      e = cudaSuccess;
+    }
+    if (e == cudaSuccess) e = passes(static_cast<T*>(d), s);
+    if (d != data) {
+      if (e == cudaSuccess) e = cudaMemcpyAsync(data, d, bytes, cudaMemcpyDeviceToDevice, s);
+      cudaFreeAsync(d, s);
+    }
+    inject_skip = -1;   // the injection lasts one execution
+    inject_polls = kPollLimit;
+    return e;
+  }
+  cudaError_t passes(T* d, cudaStream_t s) {
+    const Geom g{nx, ny, nz};
+    cudaError_t e = launch_row_pass<T>(g, kind[2], tb.t[2], d, d, 0, static_cast<const T*>(nullptr), sms, true, s);
+    const ColWait wait{tma_err, inject_polls, inject_skip};
+    for (int axis = 1; axis >= 0 && e == cudaSuccess; --axis) {
+      const int k = kind[axis];
+      if constexpr (std::is_same<T, float>::value) {
+        if (tc_on) {
+          e = tc::launch_tc_pass(nx, ny, nz, axis, k, tc_tables, d, d, tma_err, sms, s);
+          if (e != cudaErrorNotSupported) continue;
+        }
+      }
+      ColJobs<T> jobs{};
+      jobs.job[0] = ColJob<T>{d, d, nullptr, is_sine(k) ? kColIndex : kColCos};
+      e = launch_col_batch<T>(g, axis, is_forward(k), jobs, 1, tb.t[axis], nullptr, T(1), wait, false, sms, s);
+    }
     return e;
   }
 };
@@ -184,7 +195,6 @@ int quasi_r2r_execute_host(quasi_r2r_plan* p, const double* in, double* out) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->own);
   bool late = false;
   if (e == cudaSuccess) e = b->timed_out(&late);
-  quasi::MapCache::get().forget(d, static_cast<char*>(d) + n * b->elem);
   cudaFree(d);
   if (e != cudaSuccess) return set_error(QUASI_ERR_CUDA, cudaGetErrorString(e));
   if (late) return set_error(QUASI_ERR_TIMEOUT, "a tile copy did not complete within its wait limit");

@@ -71,6 +71,7 @@ template <typename T, int N, int W, bool DBL, int SLOTS>
 struct RowStage {
   using F = RowFFT<T, N, kWide<T>>;
   using FD = RowFFT<double, N, kWide<T>>;
+  static constexpr int kWarps = W;
   static constexpr bool kTwo = DBL && sizeof(T) == 4;
   static constexpr int NT = 32 * W;
   static constexpr size_t xch_bytes() {
@@ -101,6 +102,7 @@ struct RowStage {
     xd = reinterpret_cast<Cx<double>*>(sm);
     slots = reinterpret_cast<Cx<T>*>(sm + xch_bytes()) + (threadIdx.x & 31);
     __syncthreads();
+    pdl_begin();
   }
   // this lane's slot s of array a
   __device__ __forceinline__ Cx<T>& slot(int a, int s) const { return slots[(a * F::E + s) * 32]; }
@@ -139,7 +141,7 @@ struct GradientStage {
 template <int N>
 using GradientSmem = RowStage<double, N, 4, true, 1>;
 template <int N>
-__global__ void __launch_bounds__(128, stage_ctas<double, N>())
+__global__ void __launch_bounds__(GradientSmem<N>::NT, stage_ctas<double, N>())
     gradient_stage_kernel(const __grid_constant__ GradientStage a, int groups, Tables<double> tb) {
   using S = GradientSmem<N>;
   using F = typename S::F;
@@ -147,9 +149,9 @@ __global__ void __launch_bounds__(128, stage_ctas<double, N>())
   const S sh(smem_raw, tb, tb, a.vqz);
   if (a.count && blockIdx.x == 0 && threadIdx.x == 0) *a.count += 1;
   const RowWarp<double, N, true> w{int(threadIdx.x & 31)};
-  const int l = w.l(), stride = gridDim.x * 4;
+  const int l = w.l(), stride = gridDim.x * S::kWarps;
   const double q02 = a.q0 * a.q0;
-  for (int grp = blockIdx.x * 4 + (threadIdx.x >> 5); grp < groups; grp += stride) {
+  for (int grp = blockIdx.x * S::kWarps + (threadIdx.x >> 5); grp < groups; grp += stride) {
     const int rg = groups - 1 - grp;
     const size_t row = (size_t(rg) * F::ROWS + 2 * w.pencil()) * N;
     Cx<double> v[F::E];
@@ -416,16 +418,16 @@ struct NonlinearStage {
 template <typename T, int N>
 using NonlinearSmem = RowStage<T, N, 4, false, 1>;
 template <typename T, int N>
-__global__ void __launch_bounds__(128, stage_ctas<T, N>())
+__global__ void __launch_bounds__(NonlinearSmem<T, N>::NT, stage_ctas<T, N>())
     nonlinear_stage_kernel(const __grid_constant__ NonlinearStage<T> a, int groups, Tables<T> tb) {
   using S = NonlinearSmem<T, N>;
   using F = typename S::F;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const S sh(smem_raw, tb, Tables<double>{}, a.vqz);
   const RowWarp<T, N, kWide<T>> w{int(threadIdx.x & 31)};
-  const int l = w.l(), stride = gridDim.x * 4;
+  const int l = w.l(), stride = gridDim.x * S::kWarps;
   const bool quasi = a.variant == 0, pcoup = quasi && *a.nloop + 1 > a.divv_switch + 1;
-  for (int grp = blockIdx.x * 4 + (threadIdx.x >> 5); grp < groups; grp += stride) {
+  for (int grp = blockIdx.x * S::kWarps + (threadIdx.x >> 5); grp < groups; grp += stride) {
     const int rg = groups - 1 - grp;
     const size_t row = (size_t(rg) * F::ROWS + 2 * w.pencil()) * N;
     Cx<T> v[F::E];
@@ -514,8 +516,7 @@ cudaError_t launch_rows(K kern, const Geom& g, int sms, cudaStream_t s, const A&
   if (e != cudaSuccess) return e;
   constexpr int W = S::NT / 32;
   const int groups = g.nx * g.ny / S::F::ROWS;
-  kern<<<std::min(per_sm * sms, (groups + W - 1) / W), S::NT, S::bytes(), s>>>(a, groups, args...);
-  return cudaGetLastError();
+  return launch_dependent(kern, std::min(per_sm * sms, (groups + W - 1) / W), S::NT, S::bytes(), s, a, groups, args...);
 }
 
 }  // namespace quasi

@@ -126,7 +126,7 @@ cudaError_t y_passes(const StepCtx<C>& c, bool forward, const YBatch<T>& b, cons
       if (!rest.n) return cudaSuccess;
     }
   }
-  return launch_col_batch<T>(c.g, 1, forward, rest.jobs, rest.n, tb, c.vqy, T(1), c.narrow, c.sms, s);
+  return launch_col_batch<T>(c.g, 1, forward, rest.jobs, rest.n, tb, c.vqy, T(1), ColWait{c.err}, c.narrow, c.sms, s);
 }
 
 // One plain pass of a field in place along x (0), y (1) or z (2).
@@ -137,7 +137,7 @@ cudaError_t plain_pass(const StepCtx<C>& c, int axis, bool forward, T* f, const 
     return launch_row_pass<T>(c.g, forward ? E10 : E01, tb, f, f, 0, static_cast<const T*>(nullptr), c.sms, true, s);
   YBatch<T> b;
   b.add(f);
-  return launch_col_batch<T>(c.g, axis, forward, b.jobs, 1, tb, nullptr, scale, c.narrow, c.sms, s);
+  return launch_col_batch<T>(c.g, axis, forward, b.jobs, 1, tb, nullptr, scale, ColWait{c.err}, c.narrow, c.sms, s);
 }
 // Forward cosine transform in place, times scale.
 template <typename T, typename C>

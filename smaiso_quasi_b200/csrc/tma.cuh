@@ -7,9 +7,6 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <map>
-#include <mutex>
-#include <tuple>
 
 namespace quasi {
 
@@ -56,6 +53,11 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Fetches a tensor map (a kernel parameter) ahead of its first use.
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
@@ -80,8 +82,10 @@ __device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.
 __device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
-// Host side: one tensor map per (field, axis) over the field as a 3-D tensor
-// (nz, ny, nx) (innermost first), box = the pass's tile (<= 256 per dim).
+// Host side: a tensor map over a field as a 3-D tensor (nz, ny, nx) (innermost
+// first), box = the pass's tile (<= 256 per dim).  Maps are plain 128-byte
+// descriptors, encoded on the host for each launch and passed by value as
+// __grid_constant__ kernel parameters (captured into the step graphs).
 // ---------------------------------------------------------------------------
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -112,44 +116,5 @@ inline bool make_field_map(CUtensorMap* map, const void* base, int elem, int nx,
                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
-
-// Process-wide cache: maps are plain 128-byte descriptors passed by value as
-// __grid_constant__ kernel parameters (captured into the step graphs).
-class MapCache {
- public:
-  static MapCache& get() {
-    static MapCache c;
-    return c;
-  }
-  bool lookup(CUtensorMap* out, const void* base, int elem, int nx, int ny, int nz, int axis, const uint32_t box[3]) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    auto key = std::make_tuple(dev, base, elem, nx, ny, nz, axis, box[0], box[1], box[2]);
-    std::lock_guard<std::mutex> lk(mu_);
-    auto it = maps_.find(key);
-    if (it != maps_.end()) {
-      *out = it->second;
-      return true;
-    }
-    CUtensorMap m;
-    if (!make_field_map(&m, base, elem, nx, ny, nz, box)) return false;
-    maps_.emplace(key, m);
-    *out = m;
-    return true;
-  }
-  // a freed field must not be found again under a reused address
-  void forget(const void* lo, const void* hi) {
-    std::lock_guard<std::mutex> lk(mu_);
-    for (auto it = maps_.begin(); it != maps_.end();) {
-      const void* b = std::get<1>(it->first);
-      if (b >= lo && b < hi) it = maps_.erase(it);
-      else ++it;
-    }
-  }
-
- private:
-  std::mutex mu_;
-  std::map<std::tuple<int, const void*, int, int, int, int, int, uint32_t, uint32_t, uint32_t>, CUtensorMap> maps_;
-};
 
 }  // namespace quasi
