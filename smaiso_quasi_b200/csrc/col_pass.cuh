@@ -93,6 +93,17 @@ struct ColIO {
       }
     }
   }
+  // sine spectra in FFTW's order: element k at N - 1 - k
+  __device__ __forceinline__ static void load_index(const T* a, int stride0, int l, Cx<T>* v) {
+    const int stride = opaque(stride0);
+#pragma unroll
+    for (int t = 0; t < F::E; ++t) v[t] = ld2(a + unsigned((N - 1 - l - F::L * t) * stride));
+  }
+  __device__ __forceinline__ static void store_index(T* a, int stride0, int l, const Cx<T>* v) {
+    const int stride = opaque(stride0);
+#pragma unroll
+    for (int t = 0; t < F::E; ++t) st2(a + unsigned((N - 1 - l - F::L * t) * stride), v[t]);
+  }
   __device__ __forceinline__ static void store_spec(T* a, int stride0, int l, const Cx<T>* v, bool sine) {
     const int stride = opaque(stride0);
     if (!sine) {

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "engine.cuh"
+#include "r2r_grid.cuh"
 
 namespace quasi {
 
@@ -79,6 +80,10 @@ struct R2R : R2RBase {
   }
   cudaError_t passes(T* d, cudaStream_t s) {
     const Geom g{nx, ny, nz};
+    // small fields in one launch (the separate passes have the waits that the
+    // failure tests make run out)
+    if (grid_form<T>(g) && !tc_on && inject_skip < 0)
+      return launch_r2r_grid(GridPasses<T>{d, g, {kind[0], kind[1], kind[2]}, {tb.t[0], tb.t[1], tb.t[2]}}, sms, s);
     cudaError_t e = launch_row_pass<T>(g, kind[2], tb.t[2], d, d, 0, static_cast<const T*>(nullptr), sms, true, s);
     const ColWait wait{tma_err, inject_polls, inject_skip};
     for (int axis = 1; axis >= 0 && e == cudaSuccess; --axis) {
