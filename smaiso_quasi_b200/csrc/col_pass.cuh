@@ -45,12 +45,6 @@ template <int G>
 __device__ __forceinline__ ColGeom x_geom(const Geom& g) { return {g.ny * g.nz, g.nz / (2 * G), size_t(g.nz)}; }
 inline int x_tiles(const Geom& g, int G) { return g.ny * (g.nz / (2 * G)); }
 
-// The threads of a tile start fetching its N rows of 2 G elements into L2.
-template <class C, int N, int G, typename T>
-__device__ __forceinline__ void prefetch_tile(const T* a, int stride, int r) {
-  for (int n = r; n < N; n += C::THREADS) prefetch_l2(a + unsigned(n * stride), 2 * G * sizeof(T));
-}
-
 // How a spectral position is read or written along the axis.
 //   cosine: place k.  sine by mode: element k is mode N - k, element 0 nothing.
 template <typename T, int N>
@@ -494,9 +488,6 @@ __global__ void __launch_bounds__(x_cta<N, G>(), x_ctas<N>())
     const int j = tile / cg.kt, k0 = (tile - j * cg.kt) * 2 * G + 2 * w.g;
     const size_t base = j * cg.outer + k0;
     const double qy = a.x.vqy[j], qz0 = a.x.vqz[k0], qz1 = a.x.vqz[k0 + 1];
-    if (const int nt = tile + gridDim.x * x_sets<N>(); nt < tiles && !a.from_spec)
-      prefetch_tile<C, N, G>(a.in + (nt / cg.kt) * cg.outer + (nt % cg.kt) * 2 * G, opaque(cg.stride),
-                                  threadIdx.x % C::THREADS);
     Cx<double> v[FD::E];
     if (!a.from_spec) {
       IOD::load_pos(a.in + base, cg.stride, l, v, false);
@@ -568,16 +559,6 @@ __global__ void __launch_bounds__(x_cta<N, G>(), x_ctas<N>())
     const size_t base = j * cg.outer + k0;
     const double qy = a.x.vqy[j], qz0 = a.x.vqz[k0], qz1 = a.x.vqz[k0 + 1];
     const double s0 = qy * qy + qz0 * qz0, s1 = qy * qy + qz1 * qz1;
-    // this tile's state, and the next tile's N, on their way while N is transformed
-    const int r = threadIdx.x % C::THREADS;
-    if (!a.from_spec) {
-      const size_t c0 = base - 2 * w.g;
-      prefetch_tile<C, N, G>(a.psiq + c0, opaque(cg.stride), r);
-      if (quasi) prefetch_tile<C, N, G>(a.psiq_old + c0, opaque(cg.stride), r);
-      if (!first) prefetch_tile<C, N, G>(a.Nq_old + c0, opaque(cg.stride), r);
-    }
-    if (const int nt = tile + gridDim.x * x_sets<N>(); nt < tiles && !a.from_spec)
-      prefetch_tile<C, N, G>(a.in + (nt / cg.kt) * cg.outer + (nt % cg.kt) * 2 * G, opaque(cg.stride), r);
     if (!a.from_spec) {
       Cx<T> u[F::E];
       IO::load_pos(a.in + base, cg.stride, l, u, false);
@@ -725,9 +706,6 @@ __global__ void __launch_bounds__(project_cta<T, N, G>(), project_ctas<T, N, G>(
     const int b = tile / cg.kt, c00 = (tile - b * cg.kt) * 2 * G;
     const size_t base = b * cg.outer + c00 + 2 * w.g;
     const T qy = T(a.x.vqy[b]);
-    if (const int nt = tile + gridDim.x; nt < tiles && (field < 3 || !stb))
-      prefetch_tile<C, N, G>(a.in[field] + (nt / cg.kt) * cg.outer + (nt % cg.kt) * 2 * G, opaque(cg.stride),
-                             threadIdx.x % C::THREADS);
     Cx<T> v[F::E];
     if (field < 3 || !stb) {
       IO::load_pos(a.in[field] + base, cg.stride, l, v, field == 0);

@@ -205,8 +205,9 @@ struct DensityStage {
   const int* nloop;
 };
 // FP32: the advection sum takes two 8-byte slot arrays and rho a double exchange
-// buffer, 12.6 KB per warp: two CTAs of 7 warps per SM.
-template <typename T> constexpr int density_warps() { return sizeof(T) == 4 ? 7 : 4; }
+// buffer, 12.6 KB per warp.  Two CTAs of 6 warps per SM: 7 fit, but with 128
+// registers per thread the kernel spills (256^3: 230 us against 198, 5 warps 217).
+template <typename T> constexpr int density_warps() { return sizeof(T) == 4 ? 6 : 4; }
 template <typename T, int N>
 using DensitySmem = RowStage<T, N, density_warps<T>(), true, sizeof(T) == 4 ? 2 : 1>;
 template <typename T, int N>
@@ -322,7 +323,7 @@ struct StressStage {
 template <typename T, int N>
 using StressSmem = RowStage<T, N, 4, false, 1>;
 template <typename T, int N>
-__global__ void __launch_bounds__(128, stage_ctas<T, N>())
+__global__ void __launch_bounds__(128, 3)
     stress_stage_kernel(const __grid_constant__ StressStage<T> a, int groups, Tables<T> tb) {
   using S = StressSmem<T, N>;
   using F = typename S::F;
@@ -418,7 +419,7 @@ struct NonlinearStage {
 template <typename T, int N>
 using NonlinearSmem = RowStage<T, N, 4, false, 1>;
 template <typename T, int N>
-__global__ void __launch_bounds__(NonlinearSmem<T, N>::NT, stage_ctas<T, N>())
+__global__ void __launch_bounds__(NonlinearSmem<T, N>::NT, 3)
     nonlinear_stage_kernel(const __grid_constant__ NonlinearStage<T> a, int groups, Tables<T> tb) {
   using S = NonlinearSmem<T, N>;
   using F = typename S::F;
@@ -427,7 +428,14 @@ __global__ void __launch_bounds__(NonlinearSmem<T, N>::NT, stage_ctas<T, N>())
   const RowWarp<T, N, kWide<T>> w{int(threadIdx.x & 31)};
   const int l = w.l(), stride = gridDim.x * S::kWarps;
   const bool quasi = a.variant == 0, pcoup = quasi && *a.nloop + 1 > a.divv_switch + 1;
-  for (int grp = blockIdx.x * S::kWarps + (threadIdx.x >> 5); grp < groups; grp += stride) {
+  Cx<T> next[F::E];   // the field after the one at work, loaded while that is transformed
+  auto fetch = [&](int c, int g) {
+    const size_t at = (size_t(groups - 1 - g) * F::ROWS + 2 * w.pencil()) * N;
+    load_rows<F, N>((c < 3 ? a.v[c] : a.p) + at, l, next, c == 2);
+  };
+  int grp = blockIdx.x * S::kWarps + (threadIdx.x >> 5);
+  if (grp < groups) fetch(0, grp);
+  for (; grp < groups; grp += stride) {
     const int rg = groups - 1 - grp;
     const size_t row = (size_t(rg) * F::ROWS + 2 * w.pencil()) * N;
     Cx<T> v[F::E];
@@ -446,7 +454,10 @@ __global__ void __launch_bounds__(NonlinearSmem<T, N>::NT, stage_ctas<T, N>())
         prefetch_rows<F, N>(a.g[0], rg - stride, w.lane);
       }
       T* f = (c < 3 ? a.v[c] : a.p) + row;
-      load_rows<F, N>(f, l, v, c == 2);
+#pragma unroll
+      for (int i = 0; i < F::E; ++i) v[i] = next[i];
+      if (c < (quasi ? 3 : 2)) fetch(c + 1, grp);
+      else if (grp + stride < groups) fetch(0, grp + stride);
       F::inverse(w, v, sh.xb, sh.t);
       F::to_pairs(w, v, c == 2);
       if (c < 3) {
