@@ -31,6 +31,15 @@ template <typename T> constexpr bool kWide = sizeof(T) == 8;
 template <typename T, int N>
 constexpr int stage_ctas() { return sizeof(T) == 8 && RowFFT<T, N, kWide<T>>::E > 8 ? 3 : 4; }
 
+// Float stages that spill at 16 warps (128 registers) run on 12 (168 registers),
+// 1.6 times faster per round of groups (stress at 256^3: 10 rounds in 266 us
+// against 7 in 297), unless that takes as many more rounds: 96x96x192 has 1.3
+// rounds of 12 warps and one of 16 (nonlinear stage 40 us on 12).
+inline bool sixteen_warps(int groups, int sms) {
+  const int r12 = (groups + 12 * sms - 1) / (12 * sms), r16 = (groups + 16 * sms - 1) / (16 * sms);
+  return 8 * r16 < 5 * r12;
+}
+
 // A lane's pairs: pair i (< E) of its two rows, element offset from row a.
 template <class F, int N>
 __device__ __forceinline__ int pair_off(int i, int l) {
@@ -141,7 +150,7 @@ struct GradientStage {
 template <int N>
 using GradientSmem = RowStage<double, N, 4, true, 1>;
 template <int N>
-__global__ void __launch_bounds__(GradientSmem<N>::NT, stage_ctas<double, N>())
+__global__ void __launch_bounds__(GradientSmem<N>::NT, N >= 512 ? 3 : 4)
     gradient_stage_kernel(const __grid_constant__ GradientStage a, int groups, Tables<double> tb) {
   using S = GradientSmem<N>;
   using F = typename S::F;
@@ -322,8 +331,8 @@ struct StressStage {
 };
 template <typename T, int N>
 using StressSmem = RowStage<T, N, 4, false, 1>;
-template <typename T, int N>
-__global__ void __launch_bounds__(128, 3)
+template <typename T, int N, int CTAS>
+__global__ void __launch_bounds__(128, CTAS)
     stress_stage_kernel(const __grid_constant__ StressStage<T> a, int groups, Tables<T> tb) {
   using S = StressSmem<T, N>;
   using F = typename S::F;
@@ -418,8 +427,8 @@ struct NonlinearStage {
 };
 template <typename T, int N>
 using NonlinearSmem = RowStage<T, N, 4, false, 1>;
-template <typename T, int N>
-__global__ void __launch_bounds__(NonlinearSmem<T, N>::NT, 3)
+template <typename T, int N, int CTAS>
+__global__ void __launch_bounds__(NonlinearSmem<T, N>::NT, CTAS)
     nonlinear_stage_kernel(const __grid_constant__ NonlinearStage<T> a, int groups, Tables<T> tb) {
   using S = NonlinearSmem<T, N>;
   using F = typename S::F;
@@ -517,16 +526,18 @@ cudaError_t launch_nonlinear_stage(const Geom& g, const NonlinearStage<T>& a, Ta
     case 512: return call(512);              \
     default: return cudaErrorInvalidValue;   \
   }
+template <class S>
+inline int stage_groups(const Geom& g) { return g.nx * g.ny / S::F::ROWS; }
 // Launch of a stage on the shared memory layout S: the resident CTAs, at most one
 // per S::NT / 32 groups of rows.
-template <class S, class K, class A, class... Args>
+template <class S, int VARIANT = 0, class K, class A, class... Args>
 cudaError_t launch_rows(K kern, const Geom& g, int sms, cudaStream_t s, const A& a, Args... args) {
-  static std::atomic<int> cache[kMaxDevices];   // per instantiation: S and A name the kernel
+  static std::atomic<int> cache[kMaxDevices];   // per instantiation: S, A and VARIANT name the kernel
   int per_sm = 1;
   const cudaError_t e = resident_ctas(kern, S::NT, S::bytes(), cache, &per_sm);
   if (e != cudaSuccess) return e;
   constexpr int W = S::NT / 32;
-  const int groups = g.nx * g.ny / S::F::ROWS;
+  const int groups = stage_groups<S>(g);
   return launch_dependent(kern, std::min(per_sm * sms, (groups + W - 1) / W), S::NT, S::bytes(), s, a, groups, args...);
 }
 

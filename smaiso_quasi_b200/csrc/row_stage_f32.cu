@@ -5,8 +5,14 @@ namespace quasi {
 using QT = float;
 
 #define QUASI_DENSITY(N) launch_rows<DensitySmem<QT, N>>(density_stage_kernel<QT, N>, g, sms, s, a, tb, tb64)
-#define QUASI_STRESS(N) launch_rows<StressSmem<QT, N>>(stress_stage_kernel<QT, N>, g, sms, s, a, tb)
-#define QUASI_NONLINEAR(N) launch_rows<NonlinearSmem<QT, N>>(nonlinear_stage_kernel<QT, N>, g, sms, s, a, tb)
+#define QUASI_STRESS(N)                                                                          \
+  (sixteen_warps(stage_groups<StressSmem<QT, N>>(g), sms)                                         \
+       ? launch_rows<StressSmem<QT, N>, 4>(stress_stage_kernel<QT, N, 4>, g, sms, s, a, tb)       \
+       : launch_rows<StressSmem<QT, N>, 3>(stress_stage_kernel<QT, N, 3>, g, sms, s, a, tb))
+#define QUASI_NONLINEAR(N)                                                                       \
+  (sixteen_warps(stage_groups<NonlinearSmem<QT, N>>(g), sms)                                      \
+       ? launch_rows<NonlinearSmem<QT, N>, 4>(nonlinear_stage_kernel<QT, N, 4>, g, sms, s, a, tb) \
+       : launch_rows<NonlinearSmem<QT, N>, 3>(nonlinear_stage_kernel<QT, N, 3>, g, sms, s, a, tb))
 
 template <>
 cudaError_t launch_density_stage<QT>(const Geom& g, const DensityStage<QT>& a, Tables<QT> tb, Tables<double> tb64,

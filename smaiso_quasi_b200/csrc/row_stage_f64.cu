@@ -5,8 +5,10 @@ namespace quasi {
 using QT = double;
 
 #define QUASI_DENSITY(N) launch_rows<DensitySmem<QT, N>>(density_stage_kernel<QT, N>, g, sms, s, a, tb, tb64)
-#define QUASI_STRESS(N) launch_rows<StressSmem<QT, N>>(stress_stage_kernel<QT, N>, g, sms, s, a, tb)
-#define QUASI_NONLINEAR(N) launch_rows<NonlinearSmem<QT, N>>(nonlinear_stage_kernel<QT, N>, g, sms, s, a, tb)
+#define QUASI_STRESS(N) \
+  launch_rows<StressSmem<QT, N>>(stress_stage_kernel<QT, N, stage_ctas<QT, N>()>, g, sms, s, a, tb)
+#define QUASI_NONLINEAR(N) \
+  launch_rows<NonlinearSmem<QT, N>>(nonlinear_stage_kernel<QT, N, stage_ctas<QT, N>()>, g, sms, s, a, tb)
 
 template <>
 cudaError_t launch_density_stage<QT>(const Geom& g, const DensityStage<QT>& a, Tables<QT> tb, Tables<double> tb64,
