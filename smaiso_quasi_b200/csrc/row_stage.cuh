@@ -115,6 +115,15 @@ struct RowStage {
   }
   // this lane's slot s of array a
   __device__ __forceinline__ Cx<T>& slot(int a, int s) const { return slots[(a * F::E + s) * 32]; }
+  // slot array 0 in double; FP32: 16-byte slots over two arrays
+  __device__ __forceinline__ Cx<double>& wide(int s) const {
+    if constexpr (sizeof(T) == 8) {
+      return slot(0, s);
+    } else {
+      static_assert(SLOTS >= 2, "two arrays");
+      return reinterpret_cast<Cx<double>*>(slots - (threadIdx.x & 31))[s * 32 + (threadIdx.x & 31)];
+    }
+  }
   // an 8-byte slot as a double
   __device__ __forceinline__ double& dslot(int a, int s) const {
     static_assert(sizeof(T) == 4, "an 8-byte slot");
@@ -130,6 +139,7 @@ __device__ __forceinline__ void prefetch_rows(const P* f, int grp, int lane) {
   if (lane == 0) prefetch_l2(f + size_t(grp) * F::ROWS * N, F::ROWS * N * sizeof(P));
 }
 
+template <typename T> __device__ __forceinline__ Cx<T> as(Cx<double> v);
 __device__ __forceinline__ Cx<float> narrow(Cx<double> v) { return Cx<float>{float(v.x), float(v.y)}; }
 template <typename T> __device__ __forceinline__ Cx<T> as(Cx<double> v);
 template <> __device__ __forceinline__ Cx<double> as<double>(Cx<double> v) { return v; }
@@ -330,7 +340,7 @@ struct StressStage {
   int variant;
 };
 template <typename T, int N>
-using StressSmem = RowStage<T, N, 4, false, 1>;
+using StressSmem = RowStage<T, N, 4, false, sizeof(T) == 4 ? 2 : 1>;
 template <typename T, int N, int CTAS>
 __global__ void __launch_bounds__(128, CTAS)
     stress_stage_kernel(const __grid_constant__ StressStage<T> a, int groups, Tables<T> tb) {
@@ -341,22 +351,25 @@ __global__ void __launch_bounds__(128, CTAS)
   const RowWarp<T, N, kWide<T>> w{int(threadIdx.x & 31)};
   const int l = w.l(), stride = gridDim.x * 4;
   const bool quasi = a.variant == 0;
-  const T ep = T(a.ep), beta = T(a.beta), gamma = T(a.gamma);
+  const T beta = T(a.beta), gamma = T(a.gamma);
   for (int grp = blockIdx.x * 4 + (threadIdx.x >> 5); grp < groups; grp += stride) {
     const int rg = groups - 1 - grp;
     const size_t row = (size_t(rg) * F::ROWS + 2 * w.pencil()) * N;
-    Cx<T> v[F::E], lr[F::E];   // lr: rho lap; slots: rho, then rho df (or mu)
+    // FP32: lap and df, and rho in the slots (double); FP64: rho lap, and rho df in
+    // the slots.  quasi-stb: mu in the slots.
+    constexpr bool kDbl = sizeof(T) == 8;
+    Cx<T> v[F::E], lap[F::E], df[kDbl ? 1 : F::E];
 #pragma unroll 1
     for (int f = quasi ? 0 : 1; f < 5; ++f) {   // lap, df, then the three components
       if (quasi) {
         if (f == 0) {
           prefetch_rows<F, N>(a.df_s, rg, w.lane);
           prefetch_rows<F, N>(a.psi, rg, w.lane);
+          prefetch_rows<F, N>(a.rho, rg, w.lane);
         } else if (f < 4) {
           prefetch_rows<F, N>(a.ld[f - 1], rg, w.lane);
         } else if (grp + stride < groups) {
           prefetch_rows<F, N>(a.lap_s, rg - stride, w.lane);
-          prefetch_rows<F, N>(a.rho, rg - stride, w.lane);
         }
       } else if (f == 4 && grp + stride < groups) {
         prefetch_rows<F, N>(a.df_s, rg - stride, w.lane);
@@ -371,28 +384,36 @@ __global__ void __launch_bounds__(128, CTAS)
       if (f == 0) {
 #pragma unroll
         for (int i = 0; i < F::E; ++i) {
-          const Cx<T> r = as<T>(ld2(a.rho + row + pair_off<F, N>(i, l)));
-          lr[i] = Cx<T>{r.x * v[i].x, r.y * v[i].y};
-          sh.slot(0, i) = r;
+          lap[i] = v[i];
         }
       } else if (f == 1) {
 #pragma unroll
         for (int i = 0; i < F::E; ++i) {
           const size_t at = row + pair_off<F, N>(i, l);
-          const Cx<T> ps = as<T>(ld2(a.psi + at));
-          auto cube = [](T p) { return p * p * p; };
-          const Cx<T> p3{cube(ps.x), cube(ps.y)}, p5{p3.x * ps.x * ps.x, p3.y * ps.y * ps.y};
-          const Cx<T> pot{beta * p3.x - gamma * p5.x, beta * p3.y - gamma * p5.y};
+          const Cx<double> ps = ld2(a.psi + at);
           if (quasi) {
-            const Cx<T> r = sh.slot(0, i);
+            // in double: near equilibrium the terms cancel, and what is left drives
+            // the density whose time derivative is divv
+            const Cx<double> r = ld2(a.rho + at);
+            auto part = [&](double p, double rr, double d, double lp) {
+              const double p2 = p * p;
+              return T(rr * (p * (a.ep + p2 * (a.beta - a.gamma * p2)) - d - lp));
+            };
             st2(a.df + at, v[i]);
-            st2(a.base + at, Cx<T>{r.x * (ep * ps.x - v[i].x + pot.x) - lr[i].x,
-                                   r.y * (ep * ps.y - v[i].y + pot.y) - lr[i].y});
-            sh.slot(0, i) = Cx<T>{r.x * v[i].x, r.y * v[i].y};
+            st2(a.base + at, Cx<T>{part(ps.x, r.x, v[i].x, lap[i].x), part(ps.y, r.y, v[i].y, lap[i].y)});
+            if constexpr (kDbl) {
+              sh.slot(0, i) = Cx<T>{r.x * v[i].x, r.y * v[i].y};
+              lap[i] = Cx<T>{r.x * lap[i].x, r.y * lap[i].y};
+            } else {
+              sh.wide(i) = r;
+              df[i] = v[i];
+            }
           } else {
-            const Cx<T> m{v[i].x - beta * p3.x + gamma * p5.x, v[i].y - beta * p3.y + gamma * p5.y};
+            const Cx<T> p = as<T>(ps);
+            auto pot = [&](T x) { return beta * x * x * x - gamma * x * x * x * x * x; };
+            const Cx<T> m{v[i].x - pot(p.x), v[i].y - pot(p.y)};
             st2(a.df + at, m);
-            st2(a.base + at, pot);
+            st2(a.base + at, Cx<T>{pot(p.x), pot(p.y)});
             sh.slot(0, i) = m;
           }
         }
@@ -400,9 +421,18 @@ __global__ void __launch_bounds__(128, CTAS)
         const int c = f - 2;
 #pragma unroll
         for (int i = 0; i < F::E; ++i) {
-          const Cx<T> g = as<T>(ld2(a.g[c] + row + pair_off<F, N>(i, l))), rd = sh.slot(0, i);
-          if (quasi) v[i] = Cx<T>{lr[i].x * g.x - rd.x * v[i].x, lr[i].y * g.y - rd.y * v[i].y};
-          else v[i] = Cx<T>{rd.x * g.x, rd.y * g.y};
+          const Cx<double> g = ld2(a.g[c] + row + pair_off<F, N>(i, l));
+          if (quasi && kDbl) {
+            const Cx<T> rd = sh.slot(0, i);
+            v[i] = Cx<T>{T(lap[i].x * g.x - rd.x * v[i].x), T(lap[i].y * g.y - rd.y * v[i].y)};
+          } else if (quasi) {   // in double: the two products nearly cancel
+            const Cx<double> r = sh.wide(i);
+            v[i] = Cx<T>{T(r.x * (double(lap[i].x) * g.x - double(df[kDbl ? 0 : i].x) * v[i].x)),
+                         T(r.y * (double(lap[i].y) * g.y - double(df[kDbl ? 0 : i].y) * v[i].y))};
+          } else {
+            const Cx<T> m = sh.slot(0, i), gt = as<T>(g);
+            v[i] = Cx<T>{m.x * gt.x, m.y * gt.y};
+          }
         }
         F::from_pairs(w, v, c == 2);
         F::forward(w, v, sh.xb, sh.t);
@@ -426,7 +456,7 @@ struct NonlinearStage {
   const int* nloop;
 };
 template <typename T, int N>
-using NonlinearSmem = RowStage<T, N, 4, false, 1>;
+using NonlinearSmem = RowStage<T, N, 4, false, sizeof(T) == 4 ? 2 : 1>;   // v . grad psi in double
 template <typename T, int N, int CTAS>
 __global__ void __launch_bounds__(NonlinearSmem<T, N>::NT, CTAS)
     nonlinear_stage_kernel(const __grid_constant__ NonlinearStage<T> a, int groups, Tables<T> tb) {
@@ -474,9 +504,8 @@ __global__ void __launch_bounds__(NonlinearSmem<T, N>::NT, CTAS)
         for (int i = 0; i < F::E; ++i) {
           const int o = pair_off<F, N>(i, l);
           st2(f + o, v[i]);
-          const Cx<T> g = as<T>(ld2(a.g[c] + row + o));
-          const Cx<T> x{v[i].x * g.x, v[i].y * g.y};
-          sh.slot(0, i) = c ? sh.slot(0, i) + x : x;
+          const Cx<double> g = ld2(a.g[c] + row + o), x{double(v[i].x) * g.x, double(v[i].y) * g.y};
+          sh.wide(i) = c ? sh.wide(i) + x : x;
         }
       } else {
 #pragma unroll
@@ -486,17 +515,18 @@ __global__ void __launch_bounds__(NonlinearSmem<T, N>::NT, CTAS)
 #pragma unroll
     for (int i = 0; i < F::E; ++i) {
       const size_t at = row + pair_off<F, N>(i, l);
-      const Cx<T> adv = sh.slot(0, i), b = ld2(a.base + at), p = v[i];
-      Cx<T> n = b - adv;
+      const Cx<T> b = ld2(a.base + at), p = v[i];
+      const Cx<double> adv = sh.wide(i);
+      Cx<double> n{b.x - adv.x, b.y - adv.y};
       if (pcoup) {
         const Cx<T> g = ld2(a.grad + at);
-        n = n + Cx<T>{p.x * g.x, p.y * g.y};
+        n = n + Cx<double>{double(p.x) * g.x, double(p.y) * g.y};
       }
       if (!quasi) {
         const Cx<T> m = ld2(a.mu + at);
-        st2(a.dtpsi + at, Cx<T>{-m.x - adv.x, -m.y - adv.y});
+        st2(a.dtpsi + at, Cx<T>{T(-m.x - adv.x), T(-m.y - adv.y)});
       }
-      v[i] = n;
+      v[i] = as<T>(n);
     }
     F::from_pairs(w, v, false);
     F::forward(w, v, sh.xb, sh.t);
