@@ -316,6 +316,7 @@ cudaError_t launch_col_batch_g(const Geom& g, int axis, const ColJobs<T>& jobs, 
   auto kern = col_batch_kernel<T, N, G, FWD>;
   static std::atomic<int> cache[kMaxDevices];
   int per_sm = 1;
+  static_assert(S::bytes() <= kSmemPerCta);
   const cudaError_t e = resident_ctas(kern, S::NT, S::bytes(), cache, &per_sm);
   if (e != cudaSuccess) return e;
   constexpr uint32_t BN = N > 256 ? N / ((N + 255) / 256) : N;
@@ -396,13 +397,14 @@ struct UpdateX {
 // three tiles of 8 warps on 32 lanes per pencil: 217 us, bound by shared memory).
 template <int N> constexpr int x_pencils() { return N >= 512 ? 4 : 8; }
 template <int N, int G> using XTile = ColTile<N, G, false, true>;
-template <int N> constexpr int x_sets() { return 4; }
+// At N = 512 the FP32 form's second set of tables leaves room for three.
+template <typename T, int N> constexpr int x_sets() { return N >= 512 && sizeof(T) == 4 ? 3 : 4; }
 // CTAs per SM that the registers must allow
 template <int N>
 constexpr int x_ctas() {
   return N >= 192 ? 1 : N >= 96 ? 2 : N >= 64 ? 2 : 4;
 }
-template <int N, int G> constexpr int x_cta() { return x_sets<N>() * XTile<N, G>::THREADS; }
+template <typename T, int N, int G> constexpr int x_cta() { return x_sets<T, N>() * XTile<N, G>::THREADS; }
 // exchange buffer (double complex, or split: double; and float complex), then the spectrum
 template <int N, int G>
 constexpr size_t x_xch_bytes() { return (size_t(XTile<N, G>::XCH) * (XTile<N, G>::template split<double>() ? 8 : 16) + 15) / 16 * 16; }
@@ -411,7 +413,7 @@ constexpr size_t x_tile_bytes() { return x_xch_bytes<N, G>() + size_t(N) * G * s
 template <typename T, int N, int G>
 constexpr size_t x_stage_smem() {   // tables of both types, wavenumbers and filter, exchange and spectrum in double
   return PencilFFT<double, N>::table_bytes() + (sizeof(T) == 4 ? PencilFFT<float, N>::table_bytes() : 0) +
-         2 * N * sizeof(double) + size_t(x_sets<N>()) * x_tile_bytes<N, G>();
+         2 * N * sizeof(double) + size_t(x_sets<T, N>()) * x_tile_bytes<N, G>();
 }
 
 // Shared memory of an x stage, as one tile's threads see it.
@@ -420,7 +422,7 @@ struct XStage {
   using C = XTile<N, G>;
   using F = PencilFFT<T, N>;
   using FD = PencilFFT<double, N>;
-  static constexpr int NT = x_cta<N, G>();
+  static constexpr int NT = x_cta<T, N, G>();
   typename FD::Tab td;
   typename F::Tab tt;
   double *q, *f;      // wavenumbers and filter factors along x
@@ -469,7 +471,7 @@ struct XStage {
 };
 
 template <typename T, int N, int G>
-__global__ void __launch_bounds__(x_cta<N, G>(), x_ctas<N>())
+__global__ void __launch_bounds__(x_cta<T, N, G>(), x_ctas<N>())
     density_x_kernel(const __grid_constant__ DensityX<T> a, Geom geom, int tiles, Tables<double> tb64, Tables<T> tb) {
   using X = XStage<T, N, G>;
   using C = typename X::C;
@@ -484,7 +486,7 @@ __global__ void __launch_bounds__(x_cta<N, G>(), x_ctas<N>())
   const C w(threadIdx.x % C::THREADS, 1 + set);
   const int l = w.l();
   const ColGeom cg = x_geom<G>(geom);
-  for (int tile = blockIdx.x * x_sets<N>() + set; tile < tiles; tile += gridDim.x * x_sets<N>()) {
+  for (int tile = blockIdx.x * x_sets<T, N>() + set; tile < tiles; tile += gridDim.x * x_sets<T, N>()) {
     const int j = tile / cg.kt, k0 = (tile - j * cg.kt) * 2 * G + 2 * w.g;
     const size_t base = j * cg.outer + k0;
     const double qy = a.x.vqy[j], qz0 = a.x.vqz[k0], qz1 = a.x.vqz[k0 + 1];
@@ -538,7 +540,7 @@ __global__ void __launch_bounds__(x_cta<N, G>(), x_ctas<N>())
 }
 
 template <typename T, int N, int G>
-__global__ void __launch_bounds__(x_cta<N, G>(), x_ctas<N>())
+__global__ void __launch_bounds__(x_cta<T, N, G>(), x_ctas<N>())
     update_x_kernel(const __grid_constant__ UpdateX<T> a, Geom geom, int tiles, Tables<double> tb64, Tables<T> tb) {
   using X = XStage<T, N, G>;
   using C = typename X::C;
@@ -554,7 +556,7 @@ __global__ void __launch_bounds__(x_cta<N, G>(), x_ctas<N>())
   const bool quasi = a.variant == 0, first = *a.nloop == 0;
   const ColGeom cg = x_geom<G>(geom);
   const double dtd2 = a.dt / 2, dsc = dtd2 * a.scale, q02 = a.q0 * a.q0;
-  for (int tile = blockIdx.x * x_sets<N>() + set; tile < tiles; tile += gridDim.x * x_sets<N>()) {
+  for (int tile = blockIdx.x * x_sets<T, N>() + set; tile < tiles; tile += gridDim.x * x_sets<T, N>()) {
     const int j = tile / cg.kt, k0 = (tile - j * cg.kt) * 2 * G + 2 * w.g;
     const size_t base = j * cg.outer + k0;
     const double qy = a.x.vqy[j], qz0 = a.x.vqz[k0], qz1 = a.x.vqz[k0 + 1];
@@ -811,8 +813,9 @@ cudaError_t launch_project_x(const Geom& g, const ProjectX<T>& a, Tables<T> tb, 
 template <typename T, int N>
 cudaError_t launch_density_x_n(const Geom& g, const DensityX<T>& a, Tables<double> tb64, Tables<T> tb, int sms,
                                cudaStream_t s) {
-  constexpr int G = x_pencils<N>(), NT = x_cta<N, G>(), SETS = x_sets<N>();
+  constexpr int G = x_pencils<N>(), NT = x_cta<T, N, G>(), SETS = x_sets<T, N>();
   constexpr size_t smem = x_stage_smem<T, N, G>();
+  static_assert(smem <= kSmemPerCta);
   auto kern = density_x_kernel<T, N, G>;
   static std::atomic<int> cache[kMaxDevices];
   int per_sm = 1;
@@ -824,8 +827,9 @@ cudaError_t launch_density_x_n(const Geom& g, const DensityX<T>& a, Tables<doubl
 template <typename T, int N>
 cudaError_t launch_update_x_n(const Geom& g, const UpdateX<T>& a, Tables<double> tb64, Tables<T> tb, int sms,
                               cudaStream_t s) {
-  constexpr int G = x_pencils<N>(), NT = x_cta<N, G>(), SETS = x_sets<N>();
+  constexpr int G = x_pencils<N>(), NT = x_cta<T, N, G>(), SETS = x_sets<T, N>();
   constexpr size_t smem = x_stage_smem<T, N, G>();
+  static_assert(smem <= kSmemPerCta);
   auto kern = update_x_kernel<T, N, G>;
   static std::atomic<int> cache[kMaxDevices];
   int per_sm = 1;
@@ -838,6 +842,7 @@ template <typename T, int N>
 cudaError_t launch_project_x_n(const Geom& g, const ProjectX<T>& a, Tables<T> tb, int sms, cudaStream_t s) {
   constexpr int G = project_pencils<T, N>(), NT = project_cta<T, N, G>();
   constexpr size_t smem = project_smem<T, N, G>();
+  static_assert(smem <= kSmemPerCta);
   auto kern = project_x_kernel<T, N, G>;
   static std::atomic<int> cache[kMaxDevices];
   int per_sm = 1;

@@ -78,6 +78,7 @@ inline cudaError_t launch_dependent(void (*kern)(P...), int grid, int block, siz
 // Resident CTAs per SM of a kernel, its dynamic shared memory allowed; found
 // once per device and instantiation.
 constexpr int kMaxDevices = 64;
+constexpr size_t kSmemPerCta = 227 * 1024;   // the most a CTA may take
 template <class K>
 inline cudaError_t resident_ctas(K kern, int threads, size_t smem, std::atomic<int>* cache, int* out) {
   int dev = 0;
@@ -208,6 +209,7 @@ cudaError_t launch_row_pass_k(const Geom& g, Tables<T> tb, const T* src, T* dst,
   auto kern = row_pass_kernel<T, N, KIND, KS>;
   static std::atomic<int> cache[kMaxDevices];
   int per_sm = 1;
+  static_assert(row_smem<T, N>() <= kSmemPerCta);
   const cudaError_t e = resident_ctas(kern, 32 * kRowWarps, row_smem<T, N>(), cache, &per_sm);
   if (e != cudaSuccess) return e;
   const int groups = g.nx * g.ny / F::ROWS;   // nx ny is a multiple of 16, ROWS divides 16

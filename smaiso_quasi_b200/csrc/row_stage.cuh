@@ -564,6 +564,7 @@ template <class S, int VARIANT = 0, class K, class A, class... Args>
 cudaError_t launch_rows(K kern, const Geom& g, int sms, cudaStream_t s, const A& a, Args... args) {
   static std::atomic<int> cache[kMaxDevices];   // per instantiation: S, A and VARIANT name the kernel
   int per_sm = 1;
+  static_assert(S::bytes() <= kSmemPerCta);
   const cudaError_t e = resident_ctas(kern, S::NT, S::bytes(), cache, &per_sm);
   if (e != cudaSuccess) return e;
   constexpr int W = S::NT / 32;
