@@ -10,7 +10,8 @@ layers (delta = 0.5) at 256^3, 1000 steps; --workload droplet512: a smectic
 droplet (r = 0.3 L) at 512x512x512, compared after its 200 steps.
 One "step" is one time step of the whole model (24 r2r transforms plus the
 pointwise stages).  The FP32 form (float fields and transforms; psi^, psi,
-grad psi, the density chain, the update and the reductions in double) is the
+grad psi, the density chain, the sums of N and of the stress, the update and
+the reductions in double) is the
 headline when its error against the plain FP64 form after the workload's run
 is within 1e-5 relative L2 in psi, rho and v; otherwise the FP64 step is.
 Both forms are timed on the same GPU and reported, with the error.
@@ -165,9 +166,7 @@ def run_profile_case(args) -> None:
     """One engine alone (FP32: about 2.3 GB on the device, FP64 about 4.6 GB):
     W + K steps, then 1 + 3 launches of the plain pass along --axis, the case
     the committed ncu summaries capture.  The autotuner is off (its timing
-    under a profiler is not the live one): the default choices, which are the
-    ones it makes live at 256^3 (double z passes as warp tiles, the rest as
-    CTA tiles)."""
+    under a profiler is not the live one)."""
     import smaiso_quasi_b200 as q
     cfg = q.default_config("quasi", *GRID, precision=args.precision, device=0, autotune=0)
     sim = q.Simulation(cfg)
@@ -229,7 +228,7 @@ def run_gpu(args) -> None:
     pk = peaks()
     cfg32, s32 = make_sim(q, "fp32", device)
     cfg64, s64 = make_sim(q, "fp64", device)
-    # the split-BF16 tensor-core form (plain x / y passes as contractions)
+    # the split-BF16 tensor-core form (plain y passes as contractions)
     cfg16 = q.default_config("quasi", *GRID, precision="bf16x3", device=device, autotune=0)   # the form as such
     s16 = q.Simulation(cfg16)
     psi0 = q.initial_condition(cfg32, IC_KIND, seed=1234)
@@ -289,15 +288,15 @@ def run_gpu(args) -> None:
             passes[f"{name}_{prec}"] = {"us": round(ms * 1e3, 2), "gbs": round(gbs, 1),
                                         "frac": round(gbs / pk["hbm_gbs"], 4)}
     head = "fp32" if fp32_ok else "fp64"
-    top = passes[f"z_{head}"]   # the z pass: the largest share of the step in the ncu launch list
+    top = passes[f"z_{head}"]   # the bare z pass: what every row stage of the step contains
     traffic = None
     prof = ROOT / "profiles" / "traffic.json"
     if prof.exists():
         t = json.loads(prof.read_text()).get(f"z_pass_{head}_256_bytes_per_launch")
         traffic = None if t is None else int(t * n_cells / 256 ** 3)
     roofline = {"bound": "hbm", "achieved": top["gbs"], "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": top["frac"],
-                "traffic": traffic, "kernel": f"tma_zpass_kernel<{'float' if head == 'fp32' else 'double'},"
-                                              f"{GRID[2]},P,0> (plain z pass)",
+                "traffic": traffic, "kernel": f"row_pass_kernel<{'float' if head == 'fp32' else 'double'},"
+                                              f"{GRID[2]}> (plain z pass)",
                 "peak_source": pk["source"] + " (burst copy)"}
 
     def step_roof(sps, sb):
@@ -315,8 +314,8 @@ def run_gpu(args) -> None:
             "metric": METRIC, "value": round(sps, 3), "unit": "steps/s", "n_gpus": args.gpus,
             "steps": K, "warmup": W, "ms_per_step": round(ms / K, 4), "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32" if fp32_ok else "f64", "data": "synthetic",
-            "headline_form": ("fp32: float fields and transforms; psi^, psi, grad psi and the density chain in "
-                              "double" if fp32_ok else "fp64 (the FP32 form missed its error bound)"),
+            "headline_form": ("fp32: float fields and transforms; psi^, psi, grad psi, the density chain and "
+                              "the sums of N and of the stress in double" if fp32_ok else "fp64 (the FP32 form missed its error bound)"),
             "config": {"workload": WORKLOAD, "grid": list(GRID), "parallelism": f"replicas x{args.gpus}",
                        "l2": "inputs larger than L2 (~30 fields of 64-128 MiB per step)",
                        "timing": f"median of {len(win32)} (fp32) / {len(win64)} (fp64) windows of K steps"},
@@ -326,7 +325,7 @@ def run_gpu(args) -> None:
                      "step_roofline": step_roof(sps64, 8), "e2e": e2e64},
             "bf16x3": {"steps_per_s": round(args.gpus * K / (ms16 / 1e3), 3), "ms_per_step": round(ms16 / K, 4),
                        "err_vs_fp64": err16,
-                       "form": "the FP32 form with its plain x / y passes as split-BF16 tensor-core contractions"},
+                       "form": "the FP32 form with its plain y passes as split-BF16 tensor-core contractions"},
             "autotune": {"fp32": s32.tuning(), "fp64": s64.tuning()},
             "speedup_fp32_vs_fp64": round(sps32 / sps64, 3),
             "cell_updates_per_s": round(sps * n_cells, 1),

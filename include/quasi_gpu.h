@@ -52,9 +52,10 @@ enum quasi_precision {
   QUASI_PREC_FP64 = 0,     /* plain form: every field and transform in double */
   QUASI_PREC_FP32 = 1,     /* fields and transforms in float; in double: the
                               carried state psi^, psi, grad psi, the density
-                              chain (law, filter, rho, divv quotient),
-                              constants, the update and the reductions */
-  QUASI_PREC_BF16X3_TC = 2 /* the FP32 form with its plain x / y transforms of
+                              chain (law, filter, rho, divv quotient), the
+                              sums of N and of the stress, constants, the
+                              update and the reductions */
+  QUASI_PREC_BF16X3_TC = 2 /* the FP32 form with its plain y transforms of
                               length 256 as split-BF16 (three-product)
                               contractions on the tensor cores, FP32
                               accumulation; r2r plans: x / y on the tensor
@@ -96,13 +97,12 @@ typedef struct quasi_config {
   int nw;               /* points per wavelength: dx = 2 pi / (q0 nw)    */
   int divv_switch;      /* divv on after this step, p coupling one later */
   double q_pert;        /* quasi-stb growth-rate probe wavenumber Q       */
-  int autotune;         /* 1 (default): quasi_create times the candidate
-                           kernels of each tunable pass (z pass as CTA or
-                           warp tiles per type; FFT or tensor-core x / y
-                           passes in the BF16X3_TC form) on this grid and
-                           keeps the fastest, remembered per grid and
-                           device for later handles; 0: fixed defaults;
-                           2: every pass as warp tiles where it can be     */
+  int autotune;         /* 1 (default): in the BF16X3_TC form quasi_create
+                           times the y pass by FFT and on the tensor cores
+                           on this grid and keeps the faster, remembered
+                           per grid and device for later handles; 0: fixed
+                           defaults; 2: the y passes on tiles of 4 pencils
+                           (one warp's own where the length allows)        */
 } quasi_config;
 
 typedef struct quasi_handle quasi_handle;
@@ -134,9 +134,9 @@ QUASI_API int quasi_step(quasi_handle* h, int nsteps);
 QUASI_API int quasi_step_timed(quasi_handle* h, int nsteps, double* device_ms);
 
 /* The autotuner's choices for this handle: out[0] / out[1] = the float /
- * double passes that run as warp tiles (bit 0 z, bit 1 x, bit 2 y; the rest as
- * CTA tiles), out[2] = axes (bit 0 x, bit 1 y) whose plain float passes run on
- * the tensor cores (BF16X3_TC form), out[3] = 1 if the choices were measured
+ * double passes that run as one warp's own tiles (bit 0 z: always; bit 1 x, bit
+ * 2 y: autotune 2), out[2] = axes (bit 1 y) whose plain float passes run on the
+ * tensor cores (BF16X3_TC form), out[3] = 1 if the choices were measured
  * (0: defaults).  No reference counterpart. */
 QUASI_API int quasi_tuning(const quasi_handle* h, int out[4]);
 
@@ -175,7 +175,8 @@ QUASI_API int quasi_growth_rate(quasi_handle* h, double* out);
 /* Exact binary checkpoint of the carried state (psiq, psiq_old, Nq_old,
  * rhoq, rho, rho_old, v, divv, divvq, p, df, psi, psi_old, grad psi, grad rho
  * in the FP64 form, the float copies of psiq and rhoq in the FP32 form, nLoop)
- * with a checksum; a file of another grid, variant or precision is rejected.
+ * with a checksum.  What follows from psiq and rhoq is derived again when the
+ * file is loaded; a file of another grid, variant or precision is rejected.
  * The reference restarts from psi text only (quasi.cpp:692-717);
  * quasi_set_psi + quasi_init reproduce that. */
 QUASI_API int quasi_save(quasi_handle* h, const char* path);
@@ -256,15 +257,18 @@ typedef struct quasi_r2r_plan quasi_r2r_plan;
 QUASI_API int quasi_r2r_plan_create(int nx, int ny, int nz, const int kind[3], int precision, int device,
                           quasi_r2r_plan** out);
 /* data: device pointer to nx*ny*nz elements (double for FP64, float for
- * FP32); stream: a cudaStream_t or NULL for the plan's own stream. */
+ * FP32); stream: a cudaStream_t or NULL for the plan's own stream.  Data that
+ * is not 16-byte aligned (floats: 8-byte, with every length at most 256) goes
+ * through a buffer allocated in stream order. */
 QUASI_API int quasi_r2r_execute_device(quasi_r2r_plan* p, void* data, void* stream);
 /* host doubles in -> host doubles out (may alias); copies included. */
 QUASI_API int quasi_r2r_execute_host(quasi_r2r_plan* p, const double* in, double* out);
 QUASI_API int quasi_r2r_plan_destroy(quasi_r2r_plan* p);
 
 /* Fault injection for failure-detection tests (no reference counterpart: the
- * reference has no failure detection).  The plan's next execution issues no
- * copy for tile `skip_tile` of each of its TMA passes and gives every tile
+ * reference has no failure detection).  The plan's next execution runs its
+ * passes as separate launches, issues no copy for tile `skip_tile` of its x and
+ * y passes and gives every tile
  * wait `poll_limit` polls: the wait of that tile runs out, the kernel drains
  * its other copies, flags the error and returns, and the synchronising
  * execution returns QUASI_ERR_TIMEOUT (the output is then undefined).  Only

@@ -25,29 +25,23 @@
 
 namespace quasi {
 
+// 12 = 3 x 4 without twiddles (Good's prime factor mapping): with n = 4 n1 + 3 n2 and
+// k = 4 k1 + 9 k2 (mod 12), W_12^{n k} = W_3^{n1 k1} W_4^{n2 k2}.
 template <typename T> struct Dft<T, 12> {
-  // 4 x 3 split: X[k1 + 4 k2] = sum_n2 W_3^{n2 k2} W_12^{n2 k1} sum_n1 a[3 n1 + n2] W_4^{n1 k1}
   QHD static void run(Cx<T>* a) {
-    const T h = T(0.5), s = T(0.86602540378443864676372317075294);
     Cx<T> t[3][4];
 #pragma unroll
-    for (int n2 = 0; n2 < 3; ++n2) {
+    for (int n1 = 0; n1 < 3; ++n1) {
 #pragma unroll
-      for (int n1 = 0; n1 < 4; ++n1) t[n2][n1] = a[3 * n1 + n2];
-      Dft<T, 4>::run(t[n2]);
+      for (int n2 = 0; n2 < 4; ++n2) t[n1][n2] = a[(4 * n1 + 3 * n2) % 12];
+      Dft<T, 4>::run(t[n1]);
     }
-    t[1][1] = cmul(t[1][1], Cx<T>{s, -h});
-    t[1][2] = cmul(t[1][2], Cx<T>{h, -s});
-    t[1][3] = mul_mi(t[1][3]);
-    t[2][1] = cmul(t[2][1], Cx<T>{h, -s});
-    t[2][2] = cmul(t[2][2], Cx<T>{-h, -s});
-    t[2][3] = Cx<T>{-t[2][3].x, -t[2][3].y};
 #pragma unroll
-    for (int k1 = 0; k1 < 4; ++k1) {
-      Cx<T> u[3] = {t[0][k1], t[1][k1], t[2][k1]};
+    for (int k2 = 0; k2 < 4; ++k2) {
+      Cx<T> u[3] = {t[0][k2], t[1][k2], t[2][k2]};
       Dft<T, 3>::run(u);
 #pragma unroll
-      for (int k2 = 0; k2 < 3; ++k2) a[k1 + 4 * k2] = u[k2];
+      for (int k1 = 0; k1 < 3; ++k1) a[(4 * k1 + 9 * k2) % 12] = u[k1];
     }
   }
 };

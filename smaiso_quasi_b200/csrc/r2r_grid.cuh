@@ -133,11 +133,12 @@ __global__ void __launch_bounds__(kGridThreads, sizeof(T) == 8 ? 3 : 4) r2r_grid
   cols(0, a.g.nx);
 }
 
-// Whether a transform takes the one-launch form.  Lengths above 256 need tiles of
-// more threads than its CTAs have.
+// Whether the one-launch form covers a grid (lengths above 256 need tiles of more
+// threads than its CTAs have), and whether a transform takes it.
+inline bool grid_lengths(const Geom& g) { return g.nx <= 256 && g.ny <= 256 && g.nz <= 256; }
 template <typename T>
 inline bool grid_form(const Geom& g) {
-  return g.nx <= 256 && g.ny <= 256 && g.nz <= 256 && size_t(g.nx) * g.ny * g.nz * sizeof(T) <= kGridBytes;
+  return grid_lengths(g) && size_t(g.nx) * g.ny * g.nz * sizeof(T) <= kGridBytes;
 }
 
 // The transform in place; every CTA of a cooperative launch is resident.

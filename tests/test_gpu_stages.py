@@ -89,11 +89,12 @@ def test_checkpoint_resumes_the_same_step(tmp_path, precision):
         assert np.array_equal(a.field(f), b.field(f)), f
 
 
-@pytest.mark.parametrize("grid", [(64, 64, 128), (64, 128, 128), (256, 16, 256), (256, 8, 256), (8, 256, 256)])
+@pytest.mark.parametrize("grid", [(64, 64, 128), (64, 128, 128), (256, 16, 256), (256, 8, 256), (8, 256, 256), (128, 128, 128),
+                                  (16, 16, 512)])
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-14), ("fp32", 2e-6)])
 def test_transform_forms(grid, precision, tol):
-    """On both sides of the one-launch form's size, on aligned data and on data
-    one pair of floats off."""
+    """On both sides of the one-launch form's size, on aligned data and on data one
+    pair of floats or one value off."""
     import torch
 
     import smaiso_quasi_b200 as q
@@ -102,7 +103,7 @@ def test_transform_forms(grid, precision, tol):
     for plan in ("STy", "iSTx"):
         ref = qo.r2r3d(a, qo.PLAN_KINDS[plan])
         p = q.R2RPlan(*grid, plan, precision=precision)
-        for off in (0, 2) if precision == "fp32" else (0,):
+        for off in (0, 2, 1) if precision == "fp32" else (0, 1):
             buf = torch.empty(a.size + off, dtype=dt, device="cuda")
             x = buf[off:]
             x.copy_(torch.from_numpy(a.astype(np.float64 if precision == "fp64" else np.float32)).reshape(-1))
