@@ -357,9 +357,9 @@ struct XTables {
 // rho (double, z and y transformed) -> rho^ = scale CT(rho) exp(-1.57^2 q^2 8)
 // (quasi.cpp:1260-1261) -> the x-inverse of rho^ and of its gradient's spectra.
 //   DBL: out0 = x(rho^), out1 = x'(rho^) in double (grad_y, grad_z follow from out0)
-//   else out0 = x(rho^) in double and the three gradient spectra's x passes from
-//   the float copy of rho^, each with its own multiplier (applied before the
-//   transform, so float rounding is not multiplied by the wavenumber)
+//   else out0 = x(rho^) in double and the three gradient spectra's x passes in
+//   float, each with its own multiplier (in double, rounded once before the
+//   transform, so that float rounding is not multiplied by the wavenumber)
 // from_spec: take rho^ from memory and leave `in` alone (a loaded state).
 template <typename T>
 struct DensityX {
@@ -452,22 +452,6 @@ struct XStage {
     __syncthreads();
     pdl_begin();
   }
-  // the tile's spectrum in T; FP32: the same bytes, after narrow_spectrum()
-  __device__ __forceinline__ Cx<T>* spect() const { return reinterpret_cast<Cx<T>*>(spec); }
-  __device__ __forceinline__ void narrow_spectrum(const C& w) const {
-    if constexpr (sizeof(T) == 4) {
-      Cx<T> y[F::E];
-#pragma unroll
-      for (int t = 0; t < F::E; ++t) {
-        const Cx<double> v = spec[(w.l() + F::L * t) * G + w.g];
-        y[t] = Cx<T>{T(v.x), T(v.y)};
-      }
-      w.sync();
-#pragma unroll
-      for (int t = 0; t < F::E; ++t) spect()[(w.l() + F::L * t) * G + w.g] = y[t];
-      w.sync();
-    }
-  }
 };
 
 template <typename T, int N, int G>
@@ -519,17 +503,15 @@ __global__ void __launch_bounds__(x_cta<T, N, G>(), x_ctas<N>())
       IOD::store_pos((o ? a.out1 : a.out0) + base, cg.stride, l, v, o == 1);
     }
     if constexpr (!kDbl) {
-      sh.narrow_spectrum(w);
-      const T mq[3] = {T(0), T(-qy), T(-qz0)}, mq1 = T(-qz1);
 #pragma unroll 1
       for (int o = 0; o < 3; ++o) {
         Cx<T> u[F::E];
 #pragma unroll
         for (int t = 0; t < F::E; ++t) {
           const int n = IO::place(l + F::L * t, o == 0);
-          const Cx<T> y = sh.spect()[n * G + w.g];
-          const T m0 = o == 0 ? T(-sh.q[n]) : o == 1 ? mq[1] : mq[2], m1 = o == 2 ? mq1 : m0;
-          u[t] = Cx<T>{y.x * m0, y.y * m1};
+          const Cx<double> y = sh.spec[n * G + w.g];
+          const double m0 = o == 0 ? -sh.q[n] : o == 1 ? -qy : -qz0, m1 = o == 2 ? -qz1 : m0;
+          u[t] = Cx<T>{T(y.x * m0), T(y.y * m1)};
         }
         F::inverse(w, u, sh.xt, sh.tt);
         IO::store_pos((o == 0 ? a.gx : o == 1 ? a.gy : a.gz) + base, cg.stride, l, u, o == 0);
@@ -616,7 +598,6 @@ __global__ void __launch_bounds__(x_cta<T, N, G>(), x_ctas<N>())
     //   (a0 + a1 q2) (b2 q2 + bx x + bc) + c,  q2 = |q|^2, x = q_x,
     // so one copy of the code serves every output (a branch per output made the
     // kernel outgrow the instruction cache).
-    sh.narrow_spectrum(w);
 #pragma unroll 1
     for (int o = 0; o < (quasi ? 5 : 1); ++o) {
       const bool ring = o < 2, x_axis = o == 2;
@@ -629,13 +610,13 @@ __global__ void __launch_bounds__(x_cta<T, N, G>(), x_ctas<N>())
 #pragma unroll
       for (int t = 0; t < F::E; ++t) {
         const int n = t == 0 && l == 0 ? 0 : n0 + dn * t;   // (mode 0: x = 0)
-        const Cx<T> y = sh.spect()[n * G + w.g];
+        const Cx<double> y = sh.spec[n * G + w.g];
         const double x = sh.q[n], xx = x * x, bxx = bx * x;
         auto mul = [&](double s, double bc) {
           const double q2 = xx + s;
           return (a0 + a1 * q2) * (b2 * q2 + (bxx + bc)) + c;
         };
-        u[t] = Cx<T>{y.x * T(mul(s0, bc0)), y.y * T(mul(s1, bc1))};
+        u[t] = Cx<T>{T(y.x * mul(s0, bc0)), T(y.y * mul(s1, bc1))};
       }
       F::inverse(w, u, sh.xt, sh.tt);
       IO::store_pos(a.out[o] + base, cg.stride, l, u, x_axis);
