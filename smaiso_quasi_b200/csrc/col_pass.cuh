@@ -544,10 +544,16 @@ __global__ void __launch_bounds__(x_cta<T, N, G>(), x_ctas<N>())
     const double qy = a.x.vqy[j], qz0 = a.x.vqz[k0], qz1 = a.x.vqz[k0 + 1];
     const double s0 = qy * qy + qz0 * qz0, s1 = qy * qy + qz1 * qz1;
     if (!a.from_spec) {
-      Cx<T> u[F::E];
-      IO::load_pos(a.in + base, cg.stride, l, u, false);
-      F::forward(w, u, sh.xt, sh.tt);
-      IO::store_spec(a.Nq + base, cg.stride, l, u, false);
+      // in double in both forms: N^ is differenced with what it nearly balances
+      Cx<T> in[F::E];
+      IO::load_pos(a.in + base, cg.stride, l, in, false);
+      Cx<double> u[FD::E];
+#pragma unroll
+      for (int t = 0; t < FD::E; ++t) u[t] = as<double>(in[t]);
+      FD::forward(w, u, sh.xd, sh.td);
+#pragma unroll
+      for (int t = 0; t < F::E; ++t) in[t] = as<T>(u[t]);
+      IO::store_spec(a.Nq + base, cg.stride, l, in, false);
       const int stride = opaque(cg.stride);
 #pragma unroll
       for (int t = 0; t < F::E; ++t) {
@@ -555,11 +561,11 @@ __global__ void __launch_bounds__(x_cta<T, N, G>(), x_ctas<N>())
         const size_t at = base + unsigned(k * stride);
         const Cx<double> pq = ld2(a.psiq + at);
         const Cx<double> po = quasi ? ld2(a.psiq_old + at) : Cx<double>{0.0, 0.0};
-        const Cx<T> no = first ? u[t] : ld2(a.Nq_old + at);   // quasi.cpp:1936-1938
-        auto advance = [&](double s, T n, T n_old, double p, double p_old) {
+        const Cx<double> no = first ? u[t] : as<double>(ld2(a.Nq_old + at));   // quasi.cpp:1936-1938
+        auto advance = [&](double s, double n, double n_old, double p, double p_old) {
           const double d = q02 - (sh.q[k] * sh.q[k] + s);
           const double alin = a.ep - a.alpha * (d * d);
-          const double forcing = dsc * (3.0 * double(n) - double(n_old));
+          const double forcing = dsc * (3.0 * n - n_old);
           if (quasi) {
             const double c1 = 2.0 - a.dt * a.rho_m * alin, c2 = 1.5 - a.dt * a.rho_m * alin;   // quasi.cpp:886-887
             return (c1 * p - 0.5 * p_old + forcing) / c2;

@@ -41,6 +41,9 @@ __device__ __forceinline__ void st2(T* p, Cx<T> v) {
   *reinterpret_cast<typename Vec2<T>::type*>(p) = w;
 }
 
+// A pair in another type.
+template <typename T, typename U>
+__device__ __forceinline__ Cx<T> as(Cx<U> v) { return Cx<T>{T(v.x), T(v.y)}; }
 // Starts fetching `bytes` (a multiple of 16) at p (16-byte aligned) into L2.
 __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");

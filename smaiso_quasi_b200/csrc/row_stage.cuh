@@ -139,12 +139,6 @@ __device__ __forceinline__ void prefetch_rows(const P* f, int grp, int lane) {
   if (lane == 0) prefetch_l2(f + size_t(grp) * F::ROWS * N, F::ROWS * N * sizeof(P));
 }
 
-template <typename T> __device__ __forceinline__ Cx<T> as(Cx<double> v);
-__device__ __forceinline__ Cx<float> narrow(Cx<double> v) { return Cx<float>{float(v.x), float(v.y)}; }
-template <typename T> __device__ __forceinline__ Cx<T> as(Cx<double> v);
-template <> __device__ __forceinline__ Cx<double> as<double>(Cx<double> v) { return v; }
-template <> __device__ __forceinline__ Cx<float> as<float>(Cx<double> v) { return narrow(v); }
-
 // psi and grad psi (all double) from the x- and y-transformed spectra: psi and
 // grad_z from `both` (quasi.cpp:1120-1186, 1963-1965), then with `law` the z pass
 // of rho = kp sqrt(q0^2 psi^2 + |grad psi|^2) + rho_0 (quasi.cpp:1243-1247).
