@@ -393,7 +393,7 @@ struct UpdateX {
 
 // Tiles of an x stage: 8 pencils (4 at N = 512), doubles exchanged in halves: a
 // tile then takes 49 KB at N = 256 and four of 4 warps fill an SM (whole exchanges
-// leave room for three: density_x 200 us at 256^3 in the FP32 form against 180;
+// leave room for three: density_x 200 us at 256^3 in the FP32 form against 174;
 // three tiles of 8 warps on 32 lanes per pencil: 217 us, bound by shared memory).
 template <int N> constexpr int x_pencils() { return N >= 512 ? 4 : 8; }
 template <int N, int G> using XTile = ColTile<N, G, false, true>;
@@ -646,7 +646,7 @@ struct ProjectX {
   double nu, scale;
   int variant, n0;   // n0: planes per emulated MPI rank (quasi.cpp:1641-1690)
 };
-// Tiles: 8 pencils in float (at N = 256 two CTAs of 512 threads per SM, 226 us at
+// Tiles: 8 pencils in float (at N = 256 two CTAs of 512 threads per SM, 202 us at
 // 256^3; one of 1024 on 32 lanes per pencil: 268 us), 4 in double for N >= 64 and
 // at N = 512.
 template <typename T, int N> constexpr int project_pencils() {

@@ -32,8 +32,8 @@ template <typename T, int N>
 constexpr int stage_ctas() { return sizeof(T) == 8 && RowFFT<T, N, kWide<T>>::E > 8 ? 3 : 4; }
 
 // Float stages that spill at 16 warps (128 registers) run on 12 (168 registers),
-// 1.6 times faster per round of groups (stress at 256^3: 10 rounds in 266 us
-// against 7 in 297), unless that takes as many more rounds: 96x96x192 has 1.3
+// 1.6 times faster per round of groups (stress at 256^3 with its sums in float:
+// 10 rounds in 266 us against 7 in 297; in double 339), unless that takes as many more rounds: 96x96x192 has 1.3
 // rounds of 12 warps and one of 16 (nonlinear stage 40 us on 12).
 inline bool sixteen_warps(int groups, int sms) {
   const int r12 = (groups + 12 * sms - 1) / (12 * sms), r16 = (groups + 16 * sms - 1) / (16 * sms);
@@ -203,8 +203,8 @@ __global__ void __launch_bounds__(GradientSmem<N>::NT, N >= 512 ? 3 : 4)
 //   grad rho of the previous step's rho^ (quasi.cpp:1188-1232) -> |grad rho| times the pressure factor
 //   rho (quasi.cpp:1266-1268); divv after the switch (quasi.cpp:1273-1289) -> its z pass
 // The difference quotient and the advection sum are taken in double.  (One stage
-// with the stress below saved a read of rho, but left 8 warps per SM: 610 us
-// against 160 + 220 at 256^3 in the FP32 form.)
+// with the stress below saved a read of rho, but left 8 warps per SM: 610 us at
+// 256^3 in the FP32 form, against 198 and 266 apart.)
 template <typename T>
 struct DensityStage {
   const T *rdx, *rdy, *rdz;         // grad rho's spectra; FP64: rdz is the cosine spectrum of that rho
@@ -219,7 +219,7 @@ struct DensityStage {
 };
 // FP32: the advection sum takes two 8-byte slot arrays and rho a double exchange
 // buffer, 12.6 KB per warp.  Two CTAs of 6 warps per SM: 7 fit, but with 128
-// registers per thread the kernel spills (256^3: 230 us against 198, 5 warps 217).
+// registers per thread the kernel spills (256^3: 230 us against 194, 5 warps 217).
 template <typename T> constexpr int density_warps() { return sizeof(T) == 4 ? 6 : 4; }
 template <typename T, int N>
 using DensitySmem = RowStage<T, N, density_warps<T>(), true, sizeof(T) == 4 ? 2 : 1>;
