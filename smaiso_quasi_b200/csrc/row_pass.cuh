@@ -8,7 +8,7 @@
 // (one TMA landing buffer read twice, three padded round trips, staged output
 // rows) took 28.7 / 60.3 us: the double pass moved 94 bytes of shared memory per
 // element, near the 128 bytes per clock of an SM.  In registers it moves 36 (one
-// exchange, the twiddles, and shuffles): 22.0 / 48.4 us.  Sixteen lanes with 16
+// exchange, the twiddles, and shuffles): 22.9 / 48.9 us.  Sixteen lanes with 16
 // elements each (one exchange) rather than 32 with 8 (two) for that reason.
 #pragma once
 #include <cuda_runtime.h>
