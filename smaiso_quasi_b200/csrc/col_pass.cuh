@@ -373,9 +373,9 @@ struct DensityX {
 
 // psi^: N -> N^, the semi-implicit update (quasi.cpp:1944-1962,
 // quasi-stb.cpp:1946-1958), then from psi^ the x-inverse passes of the next
-// step: psi and d_x psi in double (grad_y, grad_z share the first), and in T,
-// each with its multiplier, df, lap and the three of grad lap psi (quasi) or
-// -aLin psi^ (stb).
+// step: psi and d_x psi in double (grad_y, grad_z share the first), and each with
+// its multiplier, in T, df, lap and the three of grad lap psi (quasi) or, in
+// double, sh = -aLin psi^ (stb).
 template <typename T>
 struct UpdateX {
   const T* in;
@@ -384,7 +384,8 @@ struct UpdateX {
   const double *psiq, *psiq_old;
   double* psiq_new;
   double *out0, *out1;
-  T* out[5];
+  T* out[5];      // quasi
+  double* sh;     // quasi-stb
   XTables x;
   double ep, alpha, q0, rho_m, dt, scale;
   const int* nloop;   // steps completed
@@ -586,31 +587,41 @@ __global__ void __launch_bounds__(x_cta<T, N, G>(), x_ctas<N>())
       }
     }
     w.sync();
+    // psi, d_x psi; quasi-stb: sh.  aLin grows like q^4 and psi^ concentrates on
+    // |q| = q0, so a transform of -aLin psi^ rounds relative to high modes that it
+    // has amplified, and the growth rate divides that by dt: in float sh alone was
+    // nearly all of the rates' error (2e-6 over a stability ensemble).
 #pragma unroll 1
-    for (int o = 0; o < 2; ++o) {   // psi, d_x psi
+    for (int o = 0; o < (quasi ? 2 : 3); ++o) {
       Cx<double> v[FD::E];
 #pragma unroll
       for (int t = 0; t < FD::E; ++t) {
         const int n = IOD::place(l + FD::L * t, o == 1);
         v[t] = sh.spec[n * G + w.g];
         if (o == 1) v[t] = cscale(v[t], -sh.q[n]);
+        if (o == 2) {   // quasi-stb.cpp:1019
+          auto mul = [&](double s) {
+            const double d = q02 - (sh.q[n] * sh.q[n] + s);
+            return a.alpha * (d * d) - a.ep;
+          };
+          v[t] = Cx<double>{v[t].x * mul(s0), v[t].y * mul(s1)};
+        }
       }
       FD::inverse(w, v, sh.xd, sh.td);
-      IOD::store_pos((o ? a.out1 : a.out0) + base, cg.stride, l, v, o == 1);
+      IOD::store_pos((o == 0 ? a.out0 : o == 1 ? a.out1 : a.sh) + base, cg.stride, l, v, o == 1);
     }
-    // the T fields: the multiplier of quasi.cpp:1044-1047, 1120-1186 (or
-    // quasi-stb.cpp:1019) in double, rounded once; grad lap psi is |q|^2 q_A psi^
-    // in each mode, the derivative -q_A of lap psi = -|q|^2 psi.  All of them are
-    //   (a0 + a1 q2) (b2 q2 + bx x + bc) + c,  q2 = |q|^2, x = q_x,
+    // quasi's T fields: the multiplier of quasi.cpp:1044-1047, 1120-1186 in double,
+    // rounded once; grad lap psi is |q|^2 q_A psi^ in each mode, the derivative -q_A
+    // of lap psi = -|q|^2 psi.  All of them are
+    //   (a0 + a1 q2) (b2 q2 + bx x + bc),  q2 = |q|^2, x = q_x,
     // so one copy of the code serves every output (a branch per output made the
     // kernel outgrow the instruction cache).
 #pragma unroll 1
-    for (int o = 0; o < (quasi ? 5 : 1); ++o) {
+    for (int o = 0; o < (quasi ? 5 : 0); ++o) {
       const bool ring = o < 2, x_axis = o == 2;
       const double a0 = ring ? a.alpha * q02 : 0.0, a1 = ring ? -a.alpha : 1.0;
-      const double b2 = !quasi || o == 1 ? -1.0 : 0.0, bx = x_axis ? 1.0 : 0.0;
-      const double bc0 = !quasi ? q02 : o == 0 ? 1.0 : o == 3 ? qy : o == 4 ? qz0 : 0.0;
-      const double bc1 = o == 4 ? qz1 : bc0, c = quasi ? 0.0 : -a.ep;
+      const double b2 = o == 1 ? -1.0 : 0.0, bx = x_axis ? 1.0 : 0.0;
+      const double bc0 = o == 0 ? 1.0 : o == 3 ? qy : o == 4 ? qz0 : 0.0, bc1 = o == 4 ? qz1 : bc0;
       Cx<T> u[F::E];
       const int n0 = x_axis ? N - l : l, dn = x_axis ? -F::L : F::L;
 #pragma unroll
@@ -620,7 +631,7 @@ __global__ void __launch_bounds__(x_cta<T, N, G>(), x_ctas<N>())
         const double x = sh.q[n], xx = x * x, bxx = bx * x;
         auto mul = [&](double s, double bc) {
           const double q2 = xx + s;
-          return (a0 + a1 * q2) * (b2 * q2 + (bxx + bc)) + c;
+          return (a0 + a1 * q2) * (b2 * q2 + (bxx + bc));
         };
         u[t] = Cx<T>{T(y.x * mul(s0, bc0)), T(y.y * mul(s1, bc1))};
       }

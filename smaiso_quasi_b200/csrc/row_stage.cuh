@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(32 * density_warps<T>(), sizeof(T) == 4 ? 2 : 
 //   df, and the part of N that needs neither velocity nor pressure (quasi.cpp:1905-1929)
 //   S = rho (lap grad psi - df grad lap psi) (quasi.cpp:1305-1317) -> their z passes
 // quasi-stb: mu = sh - beta psi^3 + gamma psi^5 in df's place, S = mu grad psi
-// (quasi-stb.cpp:1295-1305).
+// (quasi-stb.cpp:1295-1305); in the FP32 form a kernel of its own (StressStb).
 template <typename T>
 struct StressStage {
   const T *lap_s, *df_s;   // quasi-stb: df_s is sh's spectrum
@@ -402,12 +402,11 @@ __global__ void __launch_bounds__(128, CTAS)
               sh.wide(i) = r;
               df[i] = v[i];
             }
-          } else {
-            const Cx<T> p = as<T>(ps);
+          } else if constexpr (kDbl) {
             auto pot = [&](T x) { return beta * x * x * x - gamma * x * x * x * x * x; };
-            const Cx<T> m{v[i].x - pot(p.x), v[i].y - pot(p.y)};
+            const Cx<T> p{pot(ps.x), pot(ps.y)}, m{v[i].x - p.x, v[i].y - p.y};
             st2(a.df + at, m);
-            st2(a.base + at, Cx<T>{pot(p.x), pot(p.y)});
+            st2(a.base + at, p);
             sh.slot(0, i) = m;
           }
         }
@@ -423,15 +422,73 @@ __global__ void __launch_bounds__(128, CTAS)
             const Cx<double> r = sh.wide(i);
             v[i] = Cx<T>{T(r.x * (double(lap[i].x) * g.x - double(df[kDbl ? 0 : i].x) * v[i].x)),
                          T(r.y * (double(lap[i].y) * g.y - double(df[kDbl ? 0 : i].y) * v[i].y))};
-          } else {
-            const Cx<T> m = sh.slot(0, i), gt = as<T>(g);
-            v[i] = Cx<T>{m.x * gt.x, m.y * gt.y};
+          } else if constexpr (kDbl) {
+            const Cx<T> m = sh.slot(0, i);
+            v[i] = Cx<T>{m.x * g.x, m.y * g.y};
           }
         }
         F::from_pairs(w, v, c == 2);
         F::forward(w, v, sh.xb, sh.t);
         store_rows<F, N>(a.s[c] + row, l, v, c == 2);
       }
+    }
+  }
+}
+
+// The stress of quasi-stb in the FP32 form: sh, mu and its products with grad psi
+// in double, each result rounded once.  (mu in float would do; sh is what has to
+// be in double, see update_x_kernel.)
+struct StressStb {
+  const double *sh_s, *psi, *g[3];   // sh_s: sh's spectrum
+  float *mu, *base, *s[3];
+  const double* vqz;
+  double beta, gamma;
+};
+template <int N>
+using StressStbSmem = RowStage<float, N, 4, true, 2>;
+template <int N, int CTAS>
+__global__ void __launch_bounds__(128, CTAS)
+    stress_stb_kernel(const __grid_constant__ StressStb a, int groups, Tables<float> tb, Tables<double> tb64) {
+  using S = StressStbSmem<N>;
+  using F = typename S::F;
+  using FD = typename S::FD;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const S sh(smem_raw, tb, tb64, a.vqz);
+  const RowWarp<float, N> w{int(threadIdx.x & 31)};
+  const RowWarp<double, N> wd{w.lane};
+  const int l = w.l(), stride = gridDim.x * 4;
+  for (int grp = blockIdx.x * 4 + (threadIdx.x >> 5); grp < groups; grp += stride) {
+    const int rg = groups - 1 - grp;
+    const size_t row = (size_t(rg) * F::ROWS + 2 * w.pencil()) * N;
+    prefetch_rows<F, N>(a.psi, rg, w.lane);
+    prefetch_rows<F, N>(a.g[0], rg, w.lane);
+    Cx<double> x[FD::E];
+    load_rows<FD, N>(a.sh_s + row, l, x, false);
+    FD::inverse(wd, x, sh.xd, sh.td);
+    FD::to_pairs(wd, x, false);
+#pragma unroll
+    for (int i = 0; i < FD::E; ++i) {
+      const size_t at = row + pair_off<F, N>(i, l);
+      const Cx<double> p = ld2(a.psi + at);
+      auto pot = [&](double y) { return a.beta * y * y * y - a.gamma * y * y * y * y * y; };
+      const Cx<double> n{pot(p.x), pot(p.y)}, m{x[i].x - n.x, x[i].y - n.y};
+      st2(a.mu + at, as<float>(m));
+      st2(a.base + at, as<float>(n));
+      sh.wide(i) = m;
+    }
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+      if (c < 2) prefetch_rows<F, N>(a.g[c + 1], rg, w.lane);
+      else if (grp + stride < groups) prefetch_rows<F, N>(a.sh_s, rg - stride, w.lane);
+      Cx<float> v[F::E];
+#pragma unroll
+      for (int i = 0; i < F::E; ++i) {
+        const Cx<double> g = ld2(a.g[c] + row + pair_off<F, N>(i, l)), m = sh.wide(i);
+        v[i] = Cx<float>{float(m.x * g.x), float(m.y * g.y)};
+      }
+      F::from_pairs(w, v, c == 2);
+      F::forward(w, v, sh.xb, sh.t);
+      store_rows<F, N>(a.s[c] + row, l, v, c == 2);
     }
   }
 }
@@ -535,6 +592,8 @@ cudaError_t launch_density_stage(const Geom& g, const DensityStage<T>& a, Tables
                                  cudaStream_t s);
 template <typename T>
 cudaError_t launch_stress_stage(const Geom& g, const StressStage<T>& a, Tables<T> tb, int sms, cudaStream_t s);
+cudaError_t launch_stress_stb(const Geom& g, const StressStb& a, Tables<float> tb, Tables<double> tb64, int sms,
+                              cudaStream_t s);
 template <typename T>
 cudaError_t launch_nonlinear_stage(const Geom& g, const NonlinearStage<T>& a, Tables<T> tb, int sms, cudaStream_t s);
 

@@ -28,4 +28,19 @@ cudaError_t launch_nonlinear_stage<QT>(const Geom& g, const NonlinearStage<QT>& 
                                        cudaStream_t s) {
   QUASI_ROW_LENGTHS(g.nz, QUASI_NONLINEAR)
 }
+
+// (four CTAs fit an SM's shared memory up to N = 192)
+template <int N>
+cudaError_t stress_stb(const Geom& g, const StressStb& a, Tables<QT> tb, Tables<double> tb64, int sms, cudaStream_t s) {
+  using S = StressStbSmem<N>;
+  if constexpr (4 * S::bytes() <= kSmemPerCta)
+    if (sixteen_warps(stage_groups<S>(g), sms))
+      return launch_rows<S, 4>(stress_stb_kernel<N, 4>, g, sms, s, a, tb, tb64);
+  return launch_rows<S, 3>(stress_stb_kernel<N, 3>, g, sms, s, a, tb, tb64);
+}
+#define QUASI_STRESS_STB(N) stress_stb<N>(g, a, tb, tb64, sms, s)
+cudaError_t launch_stress_stb(const Geom& g, const StressStb& a, Tables<QT> tb, Tables<double> tb64, int sms,
+                              cudaStream_t s) {
+  QUASI_ROW_LENGTHS(g.nz, QUASI_STRESS_STB)
+}
 }  // namespace quasi

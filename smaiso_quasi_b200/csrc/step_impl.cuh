@@ -147,7 +147,8 @@ cudaError_t forward3(const StepCtx<C>& c, T* f, const AxisTables<T>& tb, cudaStr
 }
 
 // From psi^: psi and grad psi (into psi, c.gx, c.gy, c.gz), the spectra of the
-// next step's df, lap and grad lap psi (or sh), and its rho law (into law).
+// next step's df, lap and grad lap psi, and its rho law (into law).  quasi-stb: the
+// spectrum of sh in double (into lap, FP32: into law, which has no other use there).
 // update: N^ and the new psi^ first (quasi.cpp:1944-1962), and the step counter
 // after; else psi^ is taken from psiq (after the pre-loop or a checkpoint).
 template <typename T>
@@ -162,8 +163,11 @@ cudaError_t enqueue_update(const StepCtx<T>& c, const AxisTables<T>& tb, const A
   u.out0 = psi;
   u.out1 = c.gx;
   const bool quasi = c.variant == kQuasi;
-  T* outs[5] = {quasi ? c.dfs : c.lap, c.lap, c.ldx, c.ldy, c.ldz};
+  T* outs[5] = {c.dfs, c.lap, c.ldx, c.ldy, c.ldz};
   for (int o = 0; o < 5; ++o) u.out[o] = outs[o];
+  double* sh = law;
+  if constexpr (!kStateCopy<T>) sh = c.lap;
+  u.sh = sh;
   u.x = c.x;
   u.ep = c.ep; u.alpha = c.alpha; u.q0 = c.q0; u.rho_m = c.rho_m; u.dt = c.dt; u.scale = c.scale;
   u.nloop = c.nloop;
@@ -182,14 +186,14 @@ cudaError_t enqueue_update(const StepCtx<T>& c, const AxisTables<T>& tb, const A
     yt.add(c.ldy, kColSine);
     yt.add(c.ldz);
   } else {
-    yt.add(c.lap);
+    yd.add(sh);
   }
   if constexpr (!kStateCopy<T>) {
     for (int j = 0; j < yt.n; ++j) yd.jobs.job[yd.n++] = yt.jobs.job[j];
     QUASI_TRY(y_passes(c, false, yd, tb64.t[1], s));
   } else {
     QUASI_TRY(y_passes(c, false, yd, tb64.t[1], s));
-    QUASI_TRY(y_passes(c, false, yt, tb.t[1], s));
+    if (quasi) QUASI_TRY(y_passes(c, false, yt, tb.t[1], s));
   }
   GradientStage gs{psi, c.gy, c.gx, psi, c.gx, c.gy, c.gz, quasi ? law : nullptr, c.vqz, c.kp, c.q0, c.rho0,
                    update ? c.nloop : nullptr};
@@ -256,17 +260,25 @@ cudaError_t enqueue_step(const StepCtx<T>& c, const AxisTables<T>& tb, const Axi
     ys.add(c.divvq);
   }
   // a7 stress quasi.cpp:1298-1330; quasi-stb: rho == 1, divv == 0, grad rho == 0 (quasi-stb.cpp:1232)
-  StressStage<T> st{};
-  st.lap_s = c.lap; st.df_s = quasi ? c.dfs : c.lap;
-  st.ld[0] = c.ldx; st.ld[1] = c.ldy; st.ld[2] = c.ldz;
-  st.rho = c.rho_new; st.psi = c.psi;
-  st.g[0] = c.gx; st.g[1] = c.gy; st.g[2] = c.gz;
-  st.df = quasi ? c.df : c.mu; st.base = c.base;
-  st.s[0] = c.Sx; st.s[1] = c.Sy; st.s[2] = c.Sz;
-  st.ep = c.ep; st.beta = c.beta; st.gamma = c.gamma;
-  st.variant = c.variant;
-  st.vqz = c.vqz;
-  QUASI_TRY(launch_stress_stage<T>(g, st, tb.t[2], c.sms, s));
+  if constexpr (kStateCopy<T>) {
+    if (!quasi) {
+      const StressStb st{c.law, c.psi, {c.gx, c.gy, c.gz}, c.mu, c.base, {c.Sx, c.Sy, c.Sz}, c.vqz, c.beta, c.gamma};
+      QUASI_TRY(launch_stress_stb(g, st, tb.t[2], tb64.t[2], c.sms, s));
+    }
+  }
+  if (quasi || !kStateCopy<T>) {
+    StressStage<T> st{};
+    st.lap_s = c.lap; st.df_s = quasi ? c.dfs : c.lap;
+    st.ld[0] = c.ldx; st.ld[1] = c.ldy; st.ld[2] = c.ldz;
+    st.rho = c.rho_new; st.psi = c.psi;
+    st.g[0] = c.gx; st.g[1] = c.gy; st.g[2] = c.gz;
+    st.df = quasi ? c.df : c.mu; st.base = c.base;
+    st.s[0] = c.Sx; st.s[1] = c.Sy; st.s[2] = c.Sz;
+    st.ep = c.ep; st.beta = c.beta; st.gamma = c.gamma;
+    st.variant = c.variant;
+    st.vqz = c.vqz;
+    QUASI_TRY(launch_stress_stage<T>(g, st, tb.t[2], c.sms, s));
+  }
   ys.add(c.Sx);
   ys.add(c.Sy, kColSine);
   ys.add(c.Sz);
