@@ -619,6 +619,7 @@ class Engine : public EngineBase {
     for (auto& b : psi_buf_) b = dnext();
     c_.gx = dnext(); c_.gy = dnext(); c_.gz = dnext();
     for (auto& b : rho_buf_) b = dnext();
+    if (!quasi) rho_buf_[1] = rho_buf_[0];   // rho == 1: nothing writes the next step's
     law_buf_[0] = dnext();
     law_buf_[1] = kStateCopy<T> ? law_buf_[0] : dnext();
     for (auto& b : nq_buf_) b = next();

@@ -1,4 +1,5 @@
-"""quasi-stb: the precision of the FP32 form's growth rates."""
+"""quasi-stb: the precision of the FP32 form's growth rates, and rho across a
+checkpoint."""
 import math
 
 import numpy as np
@@ -34,3 +35,28 @@ def test_fp32_growth_rates():
         exact = growth_rates("fp64", seed)
         errs.append(np.linalg.norm(growth_rates("fp32", seed) - exact) / np.linalg.norm(exact))
     assert math.sqrt(np.mean(np.square(errs))) < 1e-6, errs
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("steps", [4, 5])
+def test_checkpoint_into_a_fresh_handle(tmp_path, precision, steps):
+    """rho == 1 after a load into a handle that was never initialised, whatever the
+    parity of the steps before and after it; psi bit for bit."""
+    import smaiso_quasi_b200 as q
+    cfg = q.default_config("stb", 16, 32, 64, precision=precision)
+    a = q.Simulation(cfg)
+    a.set_psi(q.initial_condition(cfg, "stb", seed=3))
+    a.init()
+    a.step(steps)
+    a.save(tmp_path / "a.bin")
+    b = q.Simulation(cfg)
+    b.load(tmp_path / "a.bin")
+    for n in range(3):
+        assert np.array_equal(b.field("psi"), a.field("psi")), n
+        assert np.all(b.field("rho") == 1.0), n
+        assert b.diagnostics()[1] == a.diagnostics()[1] > 0, n
+        a.step(1)
+        b.step(1)
+    b.save(tmp_path / "b.bin")
+    a.save(tmp_path / "a.bin")
+    assert (tmp_path / "a.bin").read_bytes() == (tmp_path / "b.bin").read_bytes()
