@@ -6,10 +6,18 @@
 #include <string>
 #include <vector>
 
+#include "col_direct.cuh"
 #include "engine.cuh"
-#include "r2r_grid.cuh"
 
 namespace quasi {
+
+// Largest field (bytes) whose column passes load and store without tensor copies
+// (col_direct.cuh).  Over grids of every length, us per transform in a graph, direct
+// against col_batch_kernel: 16x16x32 doubles 5.7 / 6.4, 64x64x128 floats 7.8 / 8.7,
+// 96x96x192 doubles 21.0 / 23.3, 128x128x256 floats (16 MB) 20.7 / 22.4; from there
+// the copies in flight tell: 128x256x256 floats 38.7 / 38.1, 256^3 74 / 67 and, in
+// double, 140 / 133.
+constexpr size_t kDirectBytes = size_t(16) << 20;
 
 struct R2RBase {
   virtual ~R2RBase() {}
@@ -57,41 +65,47 @@ struct R2R : R2RBase {
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return e;
     return cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
   }
-  // z, y, x pass in place.  The passes' tensor copies need 16-byte aligned data;
-  // pairs of floats that are 8-byte aligned go through the one-launch form whatever
-  // their size (it loads them directly), other data through a buffer allocated in
+  // z, y, x pass in place, a launch each.  (One cooperative launch for small fields
+  // saves a program with one stream 2.8 us of host time, but it needs all its CTAs
+  // resident at once: a transform of 64x64x64 floats took 12.1 us in a graph against
+  // 7.7 in three launches, 7.7 against 1.5 in one of eight branches, and 107 against
+  // 13 beside matrix products on another stream.)
+  // Tensor copies need 16-byte aligned data.  Pairs of floats that are 8-byte
+  // aligned are loaded directly, other data goes through a buffer allocated in
   // stream order.
   cudaError_t exec(void* data, cudaStream_t s) override {
-    const Geom g{nx, ny, nz};
     const size_t bytes = size_t(nx) * ny * nz * sizeof(T);
     const auto address = reinterpret_cast<uintptr_t>(data);
-    // (the failure tests make waits of the separate passes run out)
-    const bool one_launch = !tc_on && inject_skip < 0 &&
-                            (address % 16 ? address % (2 * sizeof(T)) == 0 && grid_lengths(g) : grid_form<T>(g));
+    const bool tensor = tc_on || inject_skip >= 0;   // (the failure tests make tensor copies' waits run out)
     cudaError_t e;
-    if (one_launch) {
-      e = launch_r2r_grid(GridPasses<T>{static_cast<T*>(data), g, {kind[0], kind[1], kind[2]}, {tb.t[0], tb.t[1], tb.t[2]}},
-                          sms, s);
-    } else if (address % 16) {
-      void* d = nullptr;
-      if ((e = cudaMallocAsync(&d, bytes, s)) != cudaSuccess) return e;
-      e = cudaMemcpyAsync(d, data, bytes, cudaMemcpyDeviceToDevice, s);
-      if (e == cudaSuccess) e = passes(static_cast<T*>(d), s);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(data, d, bytes, cudaMemcpyDeviceToDevice, s);
-      cudaFreeAsync(d, s);
+    if (address % 16 == 0) {
+      e = passes(static_cast<T*>(data), s, !tensor && bytes <= kDirectBytes);
+    } else if (!tensor && address % (2 * sizeof(T)) == 0 && nx <= 256 && ny <= 256 && nz <= 256) {
+      e = passes(static_cast<T*>(data), s, true);
     } else {
-      e = passes(static_cast<T*>(data), s);
+      void* d = nullptr;
+      if ((e = cudaMallocAsync(&d, bytes, s)) == cudaSuccess) {
+        e = cudaMemcpyAsync(d, data, bytes, cudaMemcpyDeviceToDevice, s);
+        if (e == cudaSuccess) e = passes(static_cast<T*>(d), s, !tensor && bytes <= kDirectBytes);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(data, d, bytes, cudaMemcpyDeviceToDevice, s);
+        cudaFreeAsync(d, s);
+      }
     }
     inject_skip = -1;   // the injection lasts one execution
     inject_polls = kPollLimit;
     return e;
   }
-  cudaError_t passes(T* d, cudaStream_t s) {
+  // direct: column passes without tensor copies
+  cudaError_t passes(T* d, cudaStream_t s, bool direct) {
     const Geom g{nx, ny, nz};
     cudaError_t e = launch_row_pass<T>(g, kind[2], tb.t[2], d, d, 0, static_cast<const T*>(nullptr), sms, true, s);
     const ColWait wait{tma_err, inject_polls, inject_skip};
     for (int axis = 1; axis >= 0 && e == cudaSuccess; --axis) {
       const int k = kind[axis];
+      if (direct) {
+        e = launch_col_direct<T>(g, axis, k, d, tb.t[axis], s);
+        continue;
+      }
       if constexpr (std::is_same<T, float>::value) {
         if (tc_on) {
           e = tc::launch_tc_pass(nx, ny, nz, axis, k, tc_tables, d, d, tma_err, sms, s);
