@@ -258,7 +258,7 @@ QUASI_API int quasi_r2r_plan_create(int nx, int ny, int nz, const int kind[3], i
                           quasi_r2r_plan** out);
 /* data: device pointer to nx*ny*nz elements (double for FP64, float for
  * FP32); stream: a cudaStream_t or NULL for the plan's own stream.  Data that
- * is not 16-byte aligned (floats: 8-byte, with every length at most 256) goes
+ * is not 16-byte aligned (floats of the FP32 form: 8-byte) goes
  * through a buffer allocated in stream order. */
 QUASI_API int quasi_r2r_execute_device(quasi_r2r_plan* p, void* data, void* stream);
 /* host doubles in -> host doubles out (may alias); copies included. */

@@ -80,7 +80,7 @@ struct R2R : R2RBase {
     cudaError_t e;
     if (address % 16 == 0) {
       e = passes(static_cast<T*>(data), s, !tensor && bytes <= kDirectBytes);
-    } else if (!tensor && address % (2 * sizeof(T)) == 0 && nx <= 256 && ny <= 256 && nz <= 256) {
+    } else if (!tensor && address % (2 * sizeof(T)) == 0) {
       e = passes(static_cast<T*>(data), s, true);
     } else {
       void* d = nullptr;
