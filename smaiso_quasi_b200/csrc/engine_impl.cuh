@@ -64,10 +64,10 @@ template <typename T>
 class Engine : public EngineBase {
  public:
   // fields of the storage type: N^ x 2, divv^, S x 3, v x 3, divv, p, df, the
-  // spectra of df, lap and grad lap psi, base, grad, grad rho's spectra x 2 (two
-  // of them in the FP64 form); double fields: psiq x 3, rhoq, psi x 2, grad psi x 3,
+  // spectra of df (then base), lap and grad lap psi, grad, grad rho's spectra x 2
+  // (two of them in the FP64 form); double fields: psiq x 3, rhoq, psi x 2, grad psi x 3,
   // rho x 2, the density scratch (x 2 in the FP64 form)
-  static constexpr int kFields = 19 + (kStateCopy<T> ? 6 : 4);
+  static constexpr int kFields = 18 + (kStateCopy<T> ? 6 : 4);
   static constexpr int kDFields = 11 + (kStateCopy<T> ? 1 : 2);
   static constexpr int kPhases = 6;   // lcm of the 3-buffer psiq and 2-buffer Nq rotations
 
@@ -440,7 +440,7 @@ class Engine : public EngineBase {
 
   int time_axis_pass(int axis, int reps, double* avg_ms) override {
     if (axis < 0 || axis > 2 || reps < 1) { err = "axis must be 0..2 and reps >= 1"; return QUASI_ERR_INVALID; }
-    T* d = c_.base;   // written and read within a step only
+    T* d = c_.Sx;   // a step writes it before it reads it
     auto one = [&]() -> cudaError_t {
       if (axis == 1) {   // as a step's y pass runs (the tensor cores in the BF16X3 form)
         YBatch<T> b;
@@ -527,7 +527,7 @@ class Engine : public EngineBase {
   // A derived field of a checkpoint, in a buffer that a step writes before it
   // reads it.
   cudaError_t derived(int which, const void** p) {
-    T* out = c_.base;
+    T* out = c_.Sx;
     *p = out;
     if constexpr (kStateCopy<T>) {
       to_storage_kernel<T><<<592, 256, 0, stream_>>>(which ? c_.rhoq : c_.psiq, out, n_);
@@ -627,7 +627,8 @@ class Engine : public EngineBase {
     c_.vx = next(); c_.vy = next(); c_.vz = next(); c_.divv = next(); c_.p = next();
     c_.df = next(); c_.dfs = next(); c_.lap = next();
     c_.ldx = next(); c_.ldy = next(); c_.ldz = next();
-    c_.base = next(); c_.grad = next();
+    c_.grad = next();
+    c_.base = c_.dfs;     // the stress stage has read df's spectrum row by row
     c_.mu = c_.lap;       // quasi-stb: mu replaces sh's spectrum row by row
     c_.dtpsi = c_.ldx;    // and has no grad lap psi
     for (auto& set : rd_buf_)

@@ -9,6 +9,24 @@ from oracle import quasi_oracle as qo
 pytestmark = pytest.mark.gpu
 
 
+def test_instance_size():
+    """Fields of a 256x256x256 instance: 24 float and 12 double ones in the FP32
+    form, 36 double ones in FP64; 16 MiB for tables, graphs and the rest."""
+    import torch
+
+    import smaiso_quasi_b200 as q
+    cells = 256 ** 3
+    q.Simulation(q.default_config("quasi", 16, 16, 32))   # the library and its kernels are loaded
+    for precision, per_cell in (("fp32", 24 * 4 + 12 * 8), ("fp64", 36 * 8)):
+        warm = q.Simulation(q.default_config("quasi", 256, 256, 256, precision=precision))
+        del warm
+        free = torch.cuda.mem_get_info()[0]
+        s = q.Simulation(q.default_config("quasi", 256, 256, 256, precision=precision))
+        used = free - torch.cuda.mem_get_info()[0]
+        del s
+        assert used <= per_cell * cells + (16 << 20), (precision, used / cells)
+
+
 def pool_high(reset=False):
     """Most bytes ever taken from the device's default memory pool."""
     cu = ctypes.CDLL("libcuda.so.1")
