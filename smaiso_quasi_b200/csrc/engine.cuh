@@ -4,17 +4,15 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include "../../include/quasi_gpu.h"
+#include "host_threads.cuh"
 #include "step_impl.cuh"
 
 namespace quasi {
@@ -50,67 +48,6 @@ class EngineBase {
 
 EngineBase* make_engine_f64(const quasi_config& cfg, std::string& err);
 EngineBase* make_engine_f32(const quasi_config& cfg, std::string& err);
-
-// Host loop over [0, n) split into contiguous chunks on up to 16 threads (the
-// field conversions between the caller's doubles and the staging buffer).
-template <class F>
-inline void host_parallel(size_t n, F&& f) {
-  unsigned hw = std::thread::hardware_concurrency();
-  const size_t nt = std::min<size_t>(hw ? hw : 1, 16);
-  if (nt <= 1 || n < (size_t(1) << 20)) {
-    f(size_t(0), n);
-    return;
-  }
-  std::vector<std::thread> pool;
-  const size_t chunk = (n + nt - 1) / nt;
-  for (size_t t = 1; t < nt; ++t) {
-    const size_t lo = std::min(n, t * chunk), hi = std::min(n, lo + chunk);
-    pool.emplace_back([&f, lo, hi] { f(lo, hi); });
-  }
-  f(size_t(0), std::min(n, chunk));
-  for (auto& th : pool) th.join();
-}
-
-// work(c) for every chunk on up to 16 threads, this one among them, each chunk
-// after arrived(c) has returned true on this thread (called in order).  A chunk
-// that does not arrive ends the loop and those after it are not worked on.
-template <class A, class W>
-inline void host_chunks(int chunks, A&& arrived, W&& work) {
-  unsigned hw = std::thread::hardware_concurrency();
-  const int nt = std::min<int>({int(hw ? hw : 1), 16, chunks});
-  std::atomic<int> ready{0}, next{0};
-  std::atomic<bool> stop{false};
-  auto drain = [&] {   // chunks that have arrived and nobody has taken
-    for (int c = next.load(); c < ready.load();) {
-      if (next.compare_exchange_weak(c, c + 1)) {
-        work(c);
-        c = next.load();
-      }
-    }
-  };
-  std::vector<std::thread> pool;
-  for (int t = 1; t < nt; ++t) {
-    try {
-      pool.emplace_back([&] {
-        while (!stop.load() && next.load() < chunks) {
-          drain();
-          std::this_thread::yield();
-        }
-      });
-    } catch (const std::system_error&) {   // no more threads: the others do the work
-      break;
-    }
-  }
-  for (int c = 0; c < chunks; ++c) {
-    if (!arrived(c)) {
-      stop.store(true);
-      break;
-    }
-    ready.store(c + 1);
-  }
-  if (!stop.load()) drain();
-  for (auto& th : pool) th.join();
-}
 
 // Validates a configuration; returns an empty string when it is usable.
 std::string validate_config(const quasi_config& c);
