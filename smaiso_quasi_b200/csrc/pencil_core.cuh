@@ -305,6 +305,7 @@ struct RowWarp {
     return Cx<T>{__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)};
   }
 };
+#endif
 
 // Columns: a tile of G pencils (2 G adjacent k) along the x or y axis on
 // THREADS = G L threads (whole warps).  A warp holds S = 32 / G values of l for
@@ -324,15 +325,16 @@ struct ColTile {
   static constexpr int XCH = ROWS * G;                    // its complex elements
   int ll, part, g, bar;
   // r: thread of the tile; bar: its named barrier
-  __device__ __forceinline__ ColTile(int r, int barrier) : bar(barrier) {
+  QHD ColTile(int r, int barrier) : bar(barrier) {
     const int lane = r & 31, sub = lane / G, h = sub % (S / 2), lo = (r / 32) * (S / 2) + h;
     g = lane % G;
     ll = sub < S / 2 ? lo : (lo == 0 ? L / 2 : L - lo);
     part = (lo == 0 ? sub : sub ^ (S / 2)) * G + g;
   }
-  __device__ __forceinline__ int l() const { return ll; }
-  __device__ __forceinline__ int partner() const { return part; }
-  __device__ __forceinline__ int at(int place) const { return place * G + g; }
+  QHD int l() const { return ll; }
+  QHD int partner() const { return part; }
+  QHD int at(int place) const { return place * G + g; }
+#ifdef __CUDACC__
   __device__ __forceinline__ void sync() const {
     if constexpr (THREADS == 32) __syncwarp();
     else asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(THREADS) : "memory");
@@ -356,7 +358,7 @@ struct ColTile {
   __device__ __forceinline__ Cx<T> shfl(Cx<T> v, int src) const {
     return Cx<T>{__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)};
   }
-};
 #endif
+};
 
 }  // namespace quasi
