@@ -1,7 +1,7 @@
 // Passes along the x and y axes on tiles of G pencils x all N rows, the pencils
-// in registers (pencil_core.cuh, ColTile): rows are loaded and stored directly
-// (2 G adjacent k per row: 64 to 128 bytes), one exchange through shared memory
-// in between.  Everything that a field goes through between two y passes runs in
+// in registers (pencil_core.cuh, ColTile): rows of 2 G adjacent k (64 to 128 bytes)
+// move by tensor copies in the batches and directly in the x stages, with one
+// exchange through shared memory in between.  Everything that a field goes through between two y passes runs in
 // one kernel:
 //   col_batch_kernel   the passes of several fields along one axis in one launch
 //   density_x_kernel   rho: forward x, the density filter, every inverse x pass
@@ -119,9 +119,9 @@ struct ColIO {
 enum ColOp : int {
   kColCos = 0,    // cosine kind
   kColSine = 1,   // sine kind, its spectrum by mode number
-  kColGrad = 2,   // (inverse) cosine spectrum c_m -> RODFT01 of the modes -q_m c_m: the derivative along the axis
-  kColBoth = 3,   // (inverse) dst = the cosine transform, dst2 = the derivative, one tile load
-  kColIndex = 4   // sine kind, its spectrum in FFTW's order (mode m at m - 1)
+  kColBoth = 2,   // (inverse) dst = the cosine transform, dst2 = RODFT01 of the modes -q_m c_m (the derivative
+                  // along the axis), one tile load
+  kColIndex = 3   // sine kind, its spectrum in FFTW's order (mode m at m - 1)
 };
 template <typename T>
 struct ColJob {
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(col_cta<N, G>(), (sizeof(T) == 8 ? 384 : 512) 
     // kColBoth: the derivative first
 #pragma unroll 1
     for (int pass = !FWD && op == kColBoth ? 0 : 1; pass < 2; ++pass) {
-      const bool grad = !FWD && (pass == 0 || op == kColGrad), sine = grad || op == kColSine || op == kColIndex;
+      const bool grad = !FWD && pass == 0, sine = grad || op == kColSine || op == kColIndex;
       const int order = sine && op != kColIndex ? N - l : N - 1 - l;   // place of a sine spectrum's element l
       Cx<T> v[F::E];
       if constexpr (FWD) {
@@ -794,8 +794,8 @@ __global__ void __launch_bounds__(project_cta<T, N, G>(), project_ctas<T, N, G>(
 // Launchers, instantiated per type in col_pass_f32.cu and col_pass_f64.cu.
 // ---------------------------------------------------------------------------
 // Passes of njobs fields along axis 0 or 1, all forward (REDFT10 / RODFT10, the
-// result times scale) or all inverse.  vq: the axis's wavenumbers (kColGrad,
-// kColBoth).  narrow: tiles of 4 pencils where that makes them one warp's.
+// result times scale) or all inverse.  vq: the axis's wavenumbers (kColBoth).
+// narrow: tiles of 4 pencils where that makes them one warp's.
 template <typename T>
 cudaError_t launch_col_batch(const Geom& g, int axis, bool forward, const ColJobs<T>& jobs, int njobs, Tables<T> tb,
                              const double* vq, T scale, const ColWait& wait, bool narrow, int sms, cudaStream_t s);

@@ -535,8 +535,8 @@ class Engine : public EngineBase {
     } else {
       if (cfg_.variant != QUASI_VARIANT_QUASI) return cudaMemsetAsync(out, 0, n_ * sizeof(T), stream_);
       if (which == 2)   // -vs_z[k] row[k + 1] of rho's spectrum
-        return launch_row_pass<T>(g_, O01, tb_.t[2], c_.law_next, out, 2, c_.vsz, sms_, true, stream_);
-      return launch_row_pass<T>(g_, E01, tb_.t[2], which ? c_.rdy : c_.rdx, out, 0, static_cast<const T*>(nullptr),
+        return launch_row_pass<T>(g_, O01, tb_.t[2], c_.law_next, out, c_.vsz, sms_, true, stream_);
+      return launch_row_pass<T>(g_, E01, tb_.t[2], which ? c_.rdy : c_.rdx, out, static_cast<const T*>(nullptr),
                                 sms_, true, stream_);
     }
   }

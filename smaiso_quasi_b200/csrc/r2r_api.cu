@@ -98,7 +98,7 @@ struct R2R : R2RBase {
   // direct: column passes without tensor copies
   cudaError_t passes(T* d, cudaStream_t s, bool direct) {
     const Geom g{nx, ny, nz};
-    cudaError_t e = launch_row_pass<T>(g, kind[2], tb.t[2], d, d, 0, static_cast<const T*>(nullptr), sms, true, s);
+    cudaError_t e = launch_row_pass<T>(g, kind[2], tb.t[2], d, d, static_cast<const T*>(nullptr), sms, true, s);
     const ColWait wait{tma_err, inject_polls, inject_skip};
     for (int axis = 1; axis >= 0 && e == cudaSuccess; --axis) {
       const int k = kind[axis];

@@ -119,19 +119,19 @@ struct RowIO {
       st2(a + N + 2 * (l + F::L * t), v[F::E - 1 - t]);
     }
   }
-  // spectral rows: v[t] = (row a, row b) at k = l + L t.  KS 1: row[k + 1] (sine
-  // kinds: the reversed input reads position N - k, nothing for k = 0); KS 2: that
-  // times -mk (mk[j] belongs to row[j + 1])
-  template <bool SINE, int KS>
+  // spectral rows: v[t] = (row a, row b) at k = l + L t.  GRAD (sine kinds): -mk[k]
+  // row[k + 1], the reversed input reads position N - k, nothing for k = 0
+  template <bool SINE, bool GRAD = false>
   __device__ __forceinline__ static void load_spec(const T* a, int l, Cx<T>* v, const T* mk = nullptr) {
-    static_assert(KS == 0 || SINE, "shifted rows are sine rows");
+    static_assert(!GRAD || SINE, "shifted rows are sine rows");
 #pragma unroll
     for (int t = 0; t < F::E; ++t) {
-      const int k = l + F::L * t, n = F::spec(k, SINE, KS != 0);
+      const int k = l + F::L * t, n = F::spec(k, SINE, GRAD);
       v[t] = Cx<T>{a[n], a[N + n]};
-      if constexpr (KS == 2) v[t] = cscale(v[t], -mk[k ? N - k - 1 : 0]);
-      if constexpr (KS != 0)
+      if constexpr (GRAD) {
+        v[t] = cscale(v[t], -mk[k ? N - k - 1 : 0]);
         if (t == 0 && k == 0) v[t] = Cx<T>{T(0), T(0)};
+      }
     }
   }
   template <bool SINE>
@@ -155,13 +155,13 @@ constexpr size_t row_smem(int warps = kRowWarps) {
 // a z pass ends on the last planes, which are still in L2.  Float kernels load
 // the next group's rows before they transform the current ones (32 more
 // registers: 23.3 -> 22.7 us at 256^3); in double the registers are the rows.
-template <typename T, int N, int KIND, int KS>
+template <typename T, int N, int KIND, bool GRAD>
 __global__ void __launch_bounds__(32 * kRowWarps, 2)
     row_pass_kernel(const T* src, T* dst, int groups, Tables<T> tb, const T* mk, int rev) {
   using F = RowFFT<T, N>;
   using IO = RowIO<T, N>;
   constexpr bool fwd = KIND == E10 || KIND == O10, sine = KIND == O10 || KIND == O01;
-  constexpr bool prefetch = sizeof(T) == 4 && KS != 2;
+  constexpr bool prefetch = sizeof(T) == 4;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5;
   Cx<T>* xb = reinterpret_cast<Cx<T>*>(smem_raw + F::table_bytes() + warp * F::xch_bytes());
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2)
   auto row = [&](int grp) { return (size_t(rev ? groups - 1 - grp : grp) * F::ROWS + 2 * w.pencil()) * N; };
   auto load = [&](int grp, Cx<T>* v) {
     if constexpr (fwd) IO::load_pairs(src + row(grp), l, v);
-    else IO::template load_spec<sine, KS>(src + row(grp), l, v, mk);
+    else IO::template load_spec<sine, GRAD>(src + row(grp), l, v, mk);
   };
   auto transform = [&](int grp, Cx<T>* v) {
     if constexpr (fwd) {
@@ -205,11 +205,11 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2)
   }
 }
 
-template <typename T, int N, int KIND, int KS>
+template <typename T, int N, int KIND, bool GRAD = false>
 cudaError_t launch_row_pass_k(const Geom& g, Tables<T> tb, const T* src, T* dst, const T* mk, int sms, bool rev,
                               cudaStream_t s) {
   using F = RowFFT<T, N>;
-  auto kern = row_pass_kernel<T, N, KIND, KS>;
+  auto kern = row_pass_kernel<T, N, KIND, GRAD>;
   static std::atomic<int> cache[kMaxDevices];
   int per_sm = 1;
   static_assert(row_smem<T, N>() <= kSmemPerCta);
@@ -221,42 +221,42 @@ cudaError_t launch_row_pass_k(const Geom& g, Tables<T> tb, const T* src, T* dst,
 }
 
 template <typename T, int N>
-cudaError_t launch_row_pass_n(const Geom& g, int kind, Tables<T> tb, const T* src, T* dst, int ks, const T* mk, int sms,
+cudaError_t launch_row_pass_n(const Geom& g, int kind, Tables<T> tb, const T* src, T* dst, const T* mk, int sms,
                               bool rev, cudaStream_t s) {
-  if (ks == 1 && kind == O01) return launch_row_pass_k<T, N, O01, 1>(g, tb, src, dst, mk, sms, rev, s);
-  if constexpr (sizeof(T) == 8) {
-    if (ks == 2 && kind == O01 && mk) return launch_row_pass_k<T, N, O01, 2>(g, tb, src, dst, mk, sms, rev, s);
+  if (mk) {
+    if constexpr (sizeof(T) == 8) {
+      if (kind == O01) return launch_row_pass_k<T, N, O01, true>(g, tb, src, dst, mk, sms, rev, s);
+    }
+    return cudaErrorNotSupported;
   }
-  if (ks) return cudaErrorNotSupported;
   switch (kind) {
-    case E10: return launch_row_pass_k<T, N, E10, 0>(g, tb, src, dst, mk, sms, rev, s);
-    case E01: return launch_row_pass_k<T, N, E01, 0>(g, tb, src, dst, mk, sms, rev, s);
-    case O10: return launch_row_pass_k<T, N, O10, 0>(g, tb, src, dst, mk, sms, rev, s);
-    default: return launch_row_pass_k<T, N, O01, 0>(g, tb, src, dst, mk, sms, rev, s);
+    case E10: return launch_row_pass_k<T, N, E10>(g, tb, src, dst, mk, sms, rev, s);
+    case E01: return launch_row_pass_k<T, N, E01>(g, tb, src, dst, mk, sms, rev, s);
+    case O10: return launch_row_pass_k<T, N, O10>(g, tb, src, dst, mk, sms, rev, s);
+    default: return launch_row_pass_k<T, N, O01>(g, tb, src, dst, mk, sms, rev, s);
   }
 }
 
-// z pass src -> dst (may be the same field).  ks: 0 plain, 1 transforms row[k + 1]
-// (zero at the top), 2 also times -mk[k] (double); ks needs kind RODFT01, other
-// combinations return cudaErrorNotSupported.  Instantiated in row_pass_f32.cu and
-// row_pass_f64.cu.
+// z pass src -> dst (may be the same field).  mk (double, RODFT01): transforms
+// -mk[k] row[k + 1], zero at the top, the z derivative of a cosine spectrum.
+// Instantiated in row_pass_f32.cu and row_pass_f64.cu.
 template <typename T>
-cudaError_t launch_row_pass(const Geom& g, int kind, Tables<T> tb, const T* src, T* dst, int ks, const T* mk, int sms,
-                            bool rev, cudaStream_t s);
+cudaError_t launch_row_pass(const Geom& g, int kind, Tables<T> tb, const T* src, T* dst, const T* mk, int sms, bool rev,
+                            cudaStream_t s);
 
 #define QUASI_INSTANTIATE_ROW_PASS(T)                                                                              \
   template <>                                                                                                      \
-  cudaError_t launch_row_pass<T>(const Geom& g, int kind, Tables<T> tb, const T* src, T* dst, int ks, const T* mk, \
+  cudaError_t launch_row_pass<T>(const Geom& g, int kind, Tables<T> tb, const T* src, T* dst, const T* mk, \
                                  int sms, bool rev, cudaStream_t s) {                                              \
     switch (g.nz) {                                                                                                \
-      case 16: return launch_row_pass_n<T, 16>(g, kind, tb, src, dst, ks, mk, sms, rev, s);                        \
-      case 32: return launch_row_pass_n<T, 32>(g, kind, tb, src, dst, ks, mk, sms, rev, s);                        \
-      case 64: return launch_row_pass_n<T, 64>(g, kind, tb, src, dst, ks, mk, sms, rev, s);                        \
-      case 96: return launch_row_pass_n<T, 96>(g, kind, tb, src, dst, ks, mk, sms, rev, s);                        \
-      case 128: return launch_row_pass_n<T, 128>(g, kind, tb, src, dst, ks, mk, sms, rev, s);                      \
-      case 192: return launch_row_pass_n<T, 192>(g, kind, tb, src, dst, ks, mk, sms, rev, s);                      \
-      case 256: return launch_row_pass_n<T, 256>(g, kind, tb, src, dst, ks, mk, sms, rev, s);                      \
-      case 512: return launch_row_pass_n<T, 512>(g, kind, tb, src, dst, ks, mk, sms, rev, s);                      \
+      case 16: return launch_row_pass_n<T, 16>(g, kind, tb, src, dst, mk, sms, rev, s);                        \
+      case 32: return launch_row_pass_n<T, 32>(g, kind, tb, src, dst, mk, sms, rev, s);                        \
+      case 64: return launch_row_pass_n<T, 64>(g, kind, tb, src, dst, mk, sms, rev, s);                        \
+      case 96: return launch_row_pass_n<T, 96>(g, kind, tb, src, dst, mk, sms, rev, s);                        \
+      case 128: return launch_row_pass_n<T, 128>(g, kind, tb, src, dst, mk, sms, rev, s);                      \
+      case 192: return launch_row_pass_n<T, 192>(g, kind, tb, src, dst, mk, sms, rev, s);                      \
+      case 256: return launch_row_pass_n<T, 256>(g, kind, tb, src, dst, mk, sms, rev, s);                      \
+      case 512: return launch_row_pass_n<T, 512>(g, kind, tb, src, dst, mk, sms, rev, s);                      \
       default: return cudaErrorNotSupported;                                                                       \
     }                                                                                                              \
   }

@@ -134,7 +134,7 @@ template <typename T, typename C>
 cudaError_t plain_pass(const StepCtx<C>& c, int axis, bool forward, T* f, const Tables<T>& tb, cudaStream_t s,
                        T scale = T(1)) {
   if (axis == 2)
-    return launch_row_pass<T>(c.g, forward ? E10 : E01, tb, f, f, 0, static_cast<const T*>(nullptr), c.sms, true, s);
+    return launch_row_pass<T>(c.g, forward ? E10 : E01, tb, f, f, static_cast<const T*>(nullptr), c.sms, true, s);
   YBatch<T> b;
   b.add(f);
   return launch_col_batch<T>(c.g, axis, forward, b.jobs, 1, tb, nullptr, scale, ColWait{c.err}, c.narrow, c.sms, s);
