@@ -32,10 +32,15 @@ template <typename T, int N>
 constexpr int stage_ctas() { return sizeof(T) == 8 && RowFFT<T, N, kWide<T>>::E > 8 ? 3 : 4; }
 
 // Float stages that spill at 16 warps (128 registers) run on 12 (168 registers),
-// 1.6 times faster per round of groups (stress at 256^3 with its sums in float:
-// 10 rounds in 266 us against 7 in 297; in double 339), unless that takes as many more rounds: 96x96x192 has 1.3
-// rounds of 12 warps and one of 16 (nonlinear stage 40 us on 12).
+// faster per round of groups (256^3: stress 10 rounds in 317 us against 7 in 434, 2.0
+// times per round; nonlinear 232 and 247 us, 1.5 times), unless that takes 8/5 as many
+// rounds: 96x96x192 has 1.3 rounds of 12 warps and one of 16 (stress 57 and 46 us,
+// nonlinear 39 and 34), 128^3 two and one (64 and 67, 45 and 38).  Sixteen have to
+// fit: at N = 512 only three CTAs of four warps do (stress of 64x64x512 70 us with
+// their registers, 95 without).
+template <class S>
 inline bool sixteen_warps(int groups, int sms) {
+  if (4 * (S::bytes() + 1024) > 228 * 1024) return false;   // an SM's shared memory; 1 KB per CTA is the system's
   const int r12 = (groups + 12 * sms - 1) / (12 * sms), r16 = (groups + 16 * sms - 1) / (16 * sms);
   return 8 * r16 < 5 * r12;
 }
