@@ -39,8 +39,8 @@ constexpr int stage_ctas() { return sizeof(T) == 8 && RowFFT<T, N, kWide<T>>::E 
 // fit: at N = 512 only three CTAs of four warps do (stress of 64x64x512 70 us with
 // their registers, 95 without).
 template <class S>
+constexpr bool kSixteenFit = 4 * (S::bytes() + 1024) <= 228 * 1024;   // an SM's shared memory, 1 KB per CTA reserved
 inline bool sixteen_warps(int groups, int sms) {
-  if (4 * (S::bytes() + 1024) > 228 * 1024) return false;   // an SM's shared memory; 1 KB per CTA is the system's
   const int r12 = (groups + 12 * sms - 1) / (12 * sms), r16 = (groups + 16 * sms - 1) / (16 * sms);
   return 8 * r16 < 5 * r12;
 }
