@@ -53,8 +53,8 @@ enum quasi_precision {
   QUASI_PREC_FP32 = 1,     /* fields and transforms in float; in double: the
                               carried state psi^, psi, grad psi, the density
                               chain (law, filter, rho, divv quotient), the
-                              sums of N and of the stress, constants, the
-                              update and the reductions */
+                              sums of N and of the stress, quasi-stb's sh,
+                              constants, the update and the reductions */
   QUASI_PREC_BF16X3_TC = 2 /* the FP32 form with its plain y transforms of
                               length 256 as split-BF16 (three-product)
                               contractions on the tensor cores, FP32
@@ -133,11 +133,13 @@ QUASI_API int quasi_step(quasi_handle* h, int nsteps);
  * *device_ms receives the elapsed device time of the nsteps steps. */
 QUASI_API int quasi_step_timed(quasi_handle* h, int nsteps, double* device_ms);
 
-/* The autotuner's choices for this handle: out[0] / out[1] = the float /
- * double passes that run as one warp's own tiles (bit 0 z: always; bit 1 x, bit
- * 2 y: autotune 2), out[2] = axes (bit 1 y) whose plain float passes run on the
- * tensor cores (BF16X3_TC form), out[3] = 1 if the choices were measured
- * (0: defaults).  No reference counterpart. */
+/* What autotune set for this handle: out[0] / out[1] = the float / double passes
+ * asked to run as one warp's own tiles (bit 0 z: always; bits 1 x and 2 y: autotune
+ * 2, whatever the lengths; they hold for the passes that are not fused into a stage
+ * and for lengths of 64, 96 and 128), out[2] = axes (bit 1 y) whose plain float
+ * passes run on the tensor cores (BF16X3_TC form), out[3] = 1 after autotune 1 (in
+ * the BF16X3_TC form out[2] was measured then; the other forms have nothing to
+ * choose), 0: defaults.  No reference counterpart. */
 QUASI_API int quasi_tuning(const quasi_handle* h, int out[4]);
 
 /* Kernel launches in one step (kernel nodes of the step's CUDA graph; the
@@ -173,10 +175,11 @@ QUASI_API int quasi_diagnostics(quasi_handle* h, double out[3]);
 QUASI_API int quasi_growth_rate(quasi_handle* h, double* out);
 
 /* Exact binary checkpoint of the carried state (psiq, psiq_old, Nq_old,
- * rhoq, rho, rho_old, v, divv, divvq, p, df, psi, psi_old, grad psi, grad rho
- * in the FP64 form, the float copies of psiq and rhoq in the FP32 form, nLoop)
- * with a checksum.  What follows from psiq and rhoq is derived again when the
- * file is loaded; a file of another grid, variant or precision is rejected.
+ * rhoq, rho twice (it is the next step's rho_old), v, divv and its z- and
+ * y-transformed spectrum, p, df, psi, psi_old, grad psi, grad rho in the FP64 form,
+ * float copies of psiq and rhoq in the FP32 form, nLoop) with a checksum.  What
+ * follows from psiq and rhoq is derived again when the file is loaded; a file of
+ * another grid, variant or precision is rejected.
  * The reference restarts from psi text only (quasi.cpp:692-717);
  * quasi_set_psi + quasi_init reproduce that. */
 QUASI_API int quasi_save(quasi_handle* h, const char* path);

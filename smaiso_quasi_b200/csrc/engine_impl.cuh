@@ -422,7 +422,7 @@ class Engine : public EngineBase {
   void note_steps(int n) override { nloop_ += n; }
   bool initialized() const override { return initialized_; }
   void tuning(int out[4]) const override {
-    // z passes always run as warp tiles (row_pass.cuh), x / y passes with autotune = 2
+    // z passes always run as warp tiles (row_pass.cuh); x and y: as asked for
     for (int d = 0; d < 2; ++d) out[d] = 1 | (cfg_.autotune == 2 ? 6 : 0);
     out[2] = tc_on_ && tune_.tc_y ? 2 : 0;
     out[3] = tune_.measured;

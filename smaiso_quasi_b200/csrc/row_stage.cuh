@@ -209,7 +209,8 @@ __global__ void __launch_bounds__(GradientSmem<N>::NT, N >= 512 ? 3 : 4)
 //   rho (quasi.cpp:1266-1268); divv after the switch (quasi.cpp:1273-1289) -> its z pass
 // The difference quotient and the advection sum are taken in double.  (One stage
 // with the stress below saved a read of rho, but left 8 warps per SM: 610 us at
-// 256^3 in the FP32 form, against 198 and 266 apart.)
+// 256^3 in the FP32 form, against 198 and 266 apart; now, with the stress's sums in
+// double, 203 and 320.)
 template <typename T>
 struct DensityStage {
   const T *rdx, *rdy, *rdz;         // grad rho's spectra; FP64: rdz is the cosine spectrum of that rho

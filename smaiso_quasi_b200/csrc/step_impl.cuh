@@ -29,8 +29,9 @@
 //
 // Templated on the storage/transform type T (double: the plain FP64 form;
 // float: the FP32 form).  Wavenumbers, spectral constants, the semi-implicit
-// update and all reductions are evaluated in double in both forms, and both
-// keep in double what the density is built from: the carried spectral state
+// update and all reductions are evaluated in double in both forms (the projection
+// takes its wavenumbers rounded to T), and both keep in double quasi-stb's sh, and
+// what the density is built from: the carried spectral state
 // psi^, psi and grad psi (and their transforms), the density law, rho^ with
 // its Gaussian filter, rho and the divv difference quotient.  The quotient
 // (rho - rho_old)/dt (quasi.cpp:1279) amplifies step-to-step rounding noise of

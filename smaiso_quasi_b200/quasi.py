@@ -222,7 +222,7 @@ class Simulation:
         return n.value
 
     def tuning(self) -> dict:
-        """The autotuner's choices (quasi_tuning)."""
+        """What autotune set (quasi_tuning); "measured": after autotune = 1."""
         out = (ctypes.c_int * 4)()
         _check(lib().quasi_tuning(self._h, out))
         names = ("z", "x", "y")
