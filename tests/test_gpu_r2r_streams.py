@@ -102,7 +102,7 @@ def test_needs_no_idle_gpu(grid, precision):
     torch.cuda.synchronize()
     held, done = torch.cuda.Event(), torch.cuda.Event()
     with torch.cuda.stream(other):
-        torch.cuda._sleep(400_000_000)   # 0.2 s
+        torch.cuda._sleep(1_000_000_000)   # half a second
         held.record()
     p.execute_device(work.data_ptr(), st.cuda_stream)
     done.record(st)
